@@ -460,6 +460,10 @@ __global__ void k_dp_count(const int* __restrict__ level, uint32_t nl, const BNo
 // first, cost = centroid offset from the node's centre along the slot's
 // diagonal, ties to the lower child then slot), boxes widened by `margin`
 // then quantised outward in double precision
+// kQSlack: grid steps kept free around every child box, for the rounding of
+// the traversal's plane offsets (qnode_test)
+constexpr double kQSlack = 0.0078125;
+
 __global__ void k_qcollapse_write(const int* __restrict__ level, uint32_t nl, const BNode* __restrict__ nodes,
                                   uint32_t n_tris, const uint32_t* __restrict__ order, const float* __restrict__ pos,
                                   const uint32_t* __restrict__ inner_off, const uint32_t* __restrict__ tri_off,
@@ -515,13 +519,24 @@ __global__ void k_qcollapse_write(const int* __restrict__ level, uint32_t nl, co
     double scale[3];
     float porg[3];
     for (int a = 0; a < 3; ++a) {
-        const double ext = k > 0 ? static_cast<double>(phi[a]) - static_cast<double>(plo[a]) : 0.0;
+        // grid step 2^x with room for the outward rounding and kQSlack on both
+        // sides; the origin lies kQSlack steps or a little more below the boxes
         int x = -126;
-        if (ext > 0.0) {
-            frexp(ext / 255.0, &x);  // ext / 255 < 2^x
-            x = max(x, -126);
+        porg[a] = 0.0f;
+        if (k > 0) {
+            const double ext = static_cast<double>(phi[a]) - static_cast<double>(plo[a]);
+            if (ext > 0.0) {
+                frexp(ext / 255.0, &x);  // ext / 255 < 2^x
+                x = max(x, -126);
+            }
+            while (true) {
+                const double step = ldexp(1.0, x);
+                porg[a] = __double2float_rd(static_cast<double>(plo[a]) - kQSlack * step);
+                if ((static_cast<double>(phi[a]) - static_cast<double>(porg[a])) / step + kQSlack <= 255.0 || x >= 100)
+                    break;
+                ++x;
+            }
         }
-        porg[a] = k > 0 ? plo[a] : 0.0f;
         ex[a] = x;
         scale[a] = ldexp(1.0, x);
     }
@@ -541,8 +556,8 @@ __global__ void k_qcollapse_write(const int* __restrict__ level, uint32_t nl, co
         if (c < 0) continue;
         for (int a = 0; a < 3; ++a) {
             const double p = static_cast<double>(porg[a]);
-            const double l = floor((static_cast<double>(lo[c][a]) - p) / scale[a]);
-            const double h = ceil((static_cast<double>(hi[c][a]) - p) / scale[a]);
+            const double l = floor((static_cast<double>(lo[c][a]) - p) / scale[a] - kQSlack);
+            const double h = ceil((static_cast<double>(hi[c][a]) - p) / scale[a] + kQSlack);
             qlo[a][t] = static_cast<uint8_t>(fmin(fmax(l, 0.0), 255.0));
             qhi[a][t] = static_cast<uint8_t>(fmin(fmax(h, 0.0), 255.0));
         }

@@ -71,23 +71,13 @@ RT_D void set_occluded(ShiftJob& j, uint32_t v) { j.hit.x = __uint_as_float(v); 
 // queue, then [nc, nc + ns) of the shadow queue, so the two queues' tails
 // (the last, slowest rays) overlap instead of running back to back.
 // Block sizes of the traversal kernel (crisb_set_trace_block, tuned by
-// crisb_autotune): resident blocks per SM chosen so every size keeps the
-// register budget of 9 x 128 threads (56 registers; 64 at 256 threads).
-// 9 resident 128-thread blocks per SM: 13.40 -> 13.25 ms of traversal per
-// 1080p frame against 8 blocks (64 registers), despite a few more spills.
+// crisb_autotune): resident blocks per SM chosen so every size has the
+// register budget of 8 x 128 threads (64 registers).  On the 1080p workload
+// 7 / 8 / 9 / 10 blocks of 128 threads render a frame in 15.47 / 15.09 / 15.09 /
+// 15.29 ms, the 256 x 256 Cornell box in 677 / 683 / 702 / 707 us.
 template <int kB>
-struct TraceShape;
-template <>
-struct TraceShape<64> {
-    static constexpr int kMinBlocks = 18;
-};
-template <>
-struct TraceShape<128> {
-    static constexpr int kMinBlocks = 9;
-};
-template <>
-struct TraceShape<256> {
-    static constexpr int kMinBlocks = 4;
+struct TraceShape {
+    static constexpr int kMinBlocks = 8 * 128 / kB;
 };
 
 template <class R, int kB, int kFmt>

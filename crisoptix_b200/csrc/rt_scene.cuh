@@ -24,8 +24,11 @@ constexpr int kTraversalStack = 64;
 // caps only bound the work of a malformed tree (the error word records it)
 constexpr uint32_t kMaxNodeVisits = 1u << 16;
 constexpr uint32_t kKnnMaxVisits = 1u << 21;
-// robust slab test: tfar *= 1 + 2*gamma(3) (Ize 2013, "Robust BVH Ray Traversal")
-constexpr float kSlabFarScale = 1.0000003576f;
+// robust slab test (Ize 2013, "Robust BVH Ray Traversal"): the far plane's t
+// times 1 + 6 * 2^-23.  A plane's t is relatively off by at most 5 * 2^-24 (the
+// subtraction, the product and the sum 2^-24 each, the approximate reciprocal
+// 2^-23), so a near and a far plane together by 10 * 2^-24.
+constexpr float kSlabFarScale = 1.0000007153f;
 
 // BVH2 node of the prefix-endpoint search structure: boxes of both children
 // + child links.  A child link >= 0 is an inner node; a negative link
@@ -61,15 +64,31 @@ struct SceneView {
     const uint4* tex_info = nullptr;
 };
 
+// A ray prepared for the box and triangle tests: the inverse direction (box
+// tests only, so an approximate reciprocal serves: the box margin covers it),
+// the axis of the largest direction component and the shear that takes the
+// direction to that axis.
 struct RayPre {
     V3 org, dir, inv;
-    int kx, ky, kz;
+    int kz;
     float sx, sy, sz;
 };
 
 RT_HD float rcp_box(float v) {
     if (fabsf(v) < 1e-30f) v = copysignf(1e-30f, v);
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+#else
     return 1.0f / v;
+#endif
+}
+
+// v with its axes rotated cyclically so that axis kz comes last
+RT_HD V3 rotate_to_z(V3 v, int kz) {
+    const bool z = kz == 2, x = kz == 0;
+    return V3{z ? v.x : (x ? v.y : v.z), z ? v.y : (x ? v.z : v.x), z ? v.z : (x ? v.x : v.y)};
 }
 
 RT_HD RayPre make_ray(V3 o, V3 d) {
@@ -84,53 +103,49 @@ RT_HD RayPre make_ray(V3 o, V3 d) {
         m = ay;
     }
     if (az > m) kz = 2;
-    int kx = kz == 2 ? 0 : kz + 1;
-    int ky = kx == 2 ? 0 : kx + 1;
-    if (comp(d, kz) < 0.0f) {
-        const int t = kx;
-        kx = ky;
-        ky = t;
-    }
-    r.kx = kx;
-    r.ky = ky;
     r.kz = kz;
-    const float dz = comp(d, kz);
-    r.sx = comp(d, kx) / dz;
-    r.sy = comp(d, ky) / dz;
-    r.sz = 1.0f / dz;
+    const V3 dr = rotate_to_z(d, kz);
+    r.sx = dr.x / dr.z;
+    r.sy = dr.y / dr.z;
+    r.sz = 1.0f / dr.z;
     r.inv = V3{rcp_box(d.x), rcp_box(d.y), rcp_box(d.z)};
     return r;
 }
 
 // Watertight ray/triangle test (Woop, Benthin & Wald, JCGT 2013).  u and v
-// are the barycentric weights of p1 and p2 (OptiX's convention).
+// are the barycentric weights of p1 and p2 (OptiX's convention).  The test
+// swaps its first two axes where the direction's largest component is
+// negative; that only negates U, V, W and the determinant (each rounding is
+// symmetric), so t, u and v do not depend on it and the swap is made only
+// where a zero's sign could: in the double-precision case.  Choosing the last
+// axis by rotation alone and testing signs through minima and maxima took a
+// rejected triangle from 125 to 80 instructions (726 to 318 cycles).
 RT_HD bool intersect_tri(const RayPre& r, V3 p0, V3 p1, V3 p2, float tmin, float tmax, float& t_out,
                          float& u_out, float& v_out) {
-    const V3 A = p0 - r.org, B = p1 - r.org, C = p2 - r.org;
-    const float akz = comp(A, r.kz), bkz = comp(B, r.kz), ckz = comp(C, r.kz);
-    const float Ax = comp(A, r.kx) - r.sx * akz;
-    const float Ay = comp(A, r.ky) - r.sy * akz;
-    const float Bx = comp(B, r.kx) - r.sx * bkz;
-    const float By = comp(B, r.ky) - r.sy * bkz;
-    const float Cx = comp(C, r.kx) - r.sx * ckz;
-    const float Cy = comp(C, r.ky) - r.sy * ckz;
+    const V3 A = rotate_to_z(p0 - r.org, r.kz), B = rotate_to_z(p1 - r.org, r.kz), C = rotate_to_z(p2 - r.org, r.kz);
+    const float Ax = A.x - r.sx * A.z;
+    const float Ay = A.y - r.sy * A.z;
+    const float Bx = B.x - r.sx * B.z;
+    const float By = B.y - r.sy * B.z;
+    const float Cx = C.x - r.sx * C.z;
+    const float Cy = C.y - r.sy * C.z;
     float U = Cx * By - Cy * Bx;
     float V = Ax * Cy - Ay * Cx;
     float W = Bx * Ay - By * Ax;
-    if (U == 0.0f || V == 0.0f || W == 0.0f) {
-        U = static_cast<float>(static_cast<double>(Cx) * static_cast<double>(By) -
-                               static_cast<double>(Cy) * static_cast<double>(Bx));
-        V = static_cast<float>(static_cast<double>(Ax) * static_cast<double>(Cy) -
-                               static_cast<double>(Ay) * static_cast<double>(Cx));
-        W = static_cast<float>(static_cast<double>(Bx) * static_cast<double>(Ay) -
-                               static_cast<double>(By) * static_cast<double>(Ax));
+    if (fminf(fminf(fabsf(U), fabsf(V)), fabsf(W)) == 0.0f) {
+        const bool swap = r.sz < 0.0f;
+        const double ax = swap ? Ay : Ax, ay = swap ? Ax : Ay, bx = swap ? By : Bx, by = swap ? Bx : By,
+                     cx = swap ? Cy : Cx, cy = swap ? Cx : Cy;
+        U = static_cast<float>(cx * by - cy * bx);
+        V = static_cast<float>(ax * cy - ay * cx);
+        W = static_cast<float>(bx * ay - by * ax);
     }
-    if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return false;
+    if (fminf(fminf(U, V), W) < 0.0f && fmaxf(fmaxf(U, V), W) > 0.0f) return false;
     const float det = U + V + W;
     if (det == 0.0f) return false;
-    const float Az = r.sz * akz;
-    const float Bz = r.sz * bkz;
-    const float Cz = r.sz * ckz;
+    const float Az = r.sz * A.z;
+    const float Bz = r.sz * B.z;
+    const float Cz = r.sz * C.z;
     const float T = U * Az + V * Bz + W * Cz;
     const float rcp_det = 1.0f / det;
     const float t = T * rcp_det;
@@ -410,6 +425,9 @@ RT_D void count_trav(const SceneView& s, uint32_t visits, uint32_t tris) {
 
 // ---- compressed 8-wide tree ------------------------------------------------------
 constexpr int kQStack = 32;
+// largest inverse direction component of the slab test: 2^15 x the largest
+// grid step (2^17 for coordinates below kQMaxCoord) x this stays finite
+constexpr float kQMaxInv = 1.9807040628566084e28f;  // 2^94
 
 // 2^e for a grid exponent e in [-126, 127]
 RT_D float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
@@ -422,11 +440,6 @@ RT_D uint64_t pk2(float lo, float hi) {
     return r;
 }
 RT_D void upk2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-RT_D uint64_t add2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 RT_D uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     uint64_t r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
@@ -443,17 +456,96 @@ RT_D float min3f(float a, float b, float c) {
     return r;
 }
 
-// Closest or first hit over the compressed tree (Bvh8QNode).  A child plane
-// at grid step q is met at t = q * (2^e * inv) + (p - o) * inv, one FMA per
-// plane on two per-node terms per axis; against the subtract-and-multiply
-// form on the decoded plane this adds roundings of |p - o| and |X - o| size,
-// far inside the box margin, so the test stays conservative and the hits are
-// those of testing every triangle (the tree only changes the speed).  Hit
-// children go into one mask: inner children at bit 24 + (slot ^ octant), leaf
-// triangles at their bits 0-23.  Inner children are taken lowest bit first
-// (near to far in the octant order); the rest of a node's hit inner children
-// wait on the stack as one group (child base, bits, inner mask, the least
-// entry t of the group, which culls the group once a closer hit is known).
+// ---- node test of the compressed tree
+// A child plane at grid step q is met at t = q * s + (p - o) * inv with
+// s = 2^e * inv.  Byte q becomes the float 2^15 + q (one byte permute: q in bits
+// 8-15 under the exponent of 2^15), so t is one FMA per plane on s and
+// b = (p - o) * inv - 2^15 * s.  Rounding b costs up to 2^-9 of a grid step
+// beside roundings of |p - o| and |X - o| size: the builder leaves kQSlack =
+// 2^-7 steps around every child box for the former and the box margin covers
+// the latter, so the test stays conservative and the hits are those of testing
+// every triangle (the tree only changes the speed).  Against bytes placed at
+// the float's low end (exact after subtracting 2^23, three packed subtractions
+// a child), per-child leaf masks and octant bits built child by child, this
+// takes 247 instead of about 330 instructions a node.
+struct QNodeHits {
+    uint32_t inner;  // hit inner children, in octant order (slot s at bit s ^ oct)
+    uint32_t leaf;   // hit leaf children, slot order
+    uint32_t child_base, tri_base, imask, meta_lo, meta_hi;
+    float tmin;      // the least entry t of the hit children
+};
+
+// meta byte of a child slot
+RT_D uint32_t qmeta(const QNodeHits& h, uint32_t slot) { return __byte_perm(h.meta_lo, h.meta_hi, slot) & 0xffu; }
+
+// inverse direction component of the compressed tree's slab test
+RT_D float qinv(float inv) { return copysignf(fminf(fabsf(inv), kQMaxInv), inv); }
+
+RT_D QNodeHits qnode_test(const Bvh8QNode* nd, V3 org, V3 inv, uint32_t oct, float tmin, float tmax) {
+    const bool ox = (oct & 1u) != 0u, oy = (oct & 2u) != 0u, oz = (oct & 4u) != 0u;
+    const float4* np = reinterpret_cast<const float4*>(nd);
+    const float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3), n4 = __ldg(np + 4);
+    const uint32_t ew = __float_as_uint(n0.w);
+    const float sx = exp2_int(static_cast<int>(static_cast<int8_t>(ew & 0xffu))) * inv.x;
+    const float sy = exp2_int(static_cast<int>(static_cast<int8_t>((ew >> 8) & 0xffu))) * inv.y;
+    const float sz = exp2_int(static_cast<int>(static_cast<int8_t>((ew >> 16) & 0xffu))) * inv.z;
+    const float bx = __fmaf_rn(-32768.0f, sx, (n0.x - org.x) * inv.x);
+    const float by = __fmaf_rn(-32768.0f, sy, (n0.y - org.y) * inv.y);
+    const float bz = __fmaf_rn(-32768.0f, sz, (n0.z - org.z) * inv.z);
+    // per axis (near, far) pairs share the scale and the offset
+    const uint64_t sx2 = pk2(sx, sx), sy2 = pk2(sy, sy), sz2 = pk2(sz, sz);
+    const uint64_t bx2 = pk2(bx, bx), by2 = pk2(by, by), bz2 = pk2(bz, bz);
+    uint32_t hits = 0;
+    float gmin = INFINITY;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t lx = __float_as_uint(h ? n2.y : n2.x), hx = __float_as_uint(h ? n3.w : n3.z);
+        const uint32_t ly = __float_as_uint(h ? n2.w : n2.z), hy = __float_as_uint(h ? n4.y : n4.x);
+        const uint32_t lz = __float_as_uint(h ? n3.y : n3.x), hz = __float_as_uint(h ? n4.w : n4.z);
+        const uint32_t nx = ox ? hx : lx, fx = ox ? lx : hx;
+        const uint32_t ny = oy ? hy : ly, fy = oy ? ly : hy;
+        const uint32_t nz = oz ? hz : lz, fz = oz ? lz : hz;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            // byte j of the near and far words as the floats 2^15 + q
+            const uint32_t sel = 0x7404u + (static_cast<uint32_t>(j) << 4);
+            float tnx, tfx, tny, tfy, tnz, tfz;
+            upk2(fma2(pk2(__uint_as_float(__byte_perm(nx, 0x47000000u, sel)),
+                          __uint_as_float(__byte_perm(fx, 0x47000000u, sel))), sx2, bx2), tnx, tfx);
+            upk2(fma2(pk2(__uint_as_float(__byte_perm(ny, 0x47000000u, sel)),
+                          __uint_as_float(__byte_perm(fy, 0x47000000u, sel))), sy2, by2), tny, tfy);
+            upk2(fma2(pk2(__uint_as_float(__byte_perm(nz, 0x47000000u, sel)),
+                          __uint_as_float(__byte_perm(fz, 0x47000000u, sel))), sz2, bz2), tnz, tfz);
+            const float tn = max3f(tnx, tny, fmaxf(tnz, tmin));
+            const float tf = min3f(tfx, tfy, fminf(tfz, tmax));
+            if (tn <= tf * kSlabFarScale) {
+                hits |= 1u << (4 * h + j);
+                gmin = fminf(gmin, tn);
+            }
+        }
+    }
+    QNodeHits r;
+    r.imask = ew >> 24;
+    uint32_t in = hits & r.imask;
+    r.leaf = hits & ~r.imask;
+    // slot s to bit s ^ oct
+    if (ox) in = ((in & 0x55u) << 1) | ((in >> 1) & 0x55u);
+    if (oy) in = ((in & 0x33u) << 2) | ((in >> 2) & 0x33u);
+    if (oz) in = ((in & 0x0fu) << 4) | (in >> 4);
+    r.inner = in;
+    r.child_base = __float_as_uint(n1.x);
+    r.tri_base = __float_as_uint(n1.y);
+    r.meta_lo = __float_as_uint(n1.z);
+    r.meta_hi = __float_as_uint(n1.w);
+    r.tmin = gmin;
+    return r;
+}
+
+// Closest or first hit over the compressed tree (Bvh8QNode).  Inner children
+// are taken lowest bit first (near to far in the octant order); the rest of a
+// node's hit inner children wait on the stack as one group (child base, bits,
+// inner mask, the least entry t of the node's hit children, which culls the
+// group once a closer hit is known).
 // Traversal state of one ray over the compressed tree; step() visits one
 // node (its eight child boxes, then the triangles of its hit leaf children)
 // and picks the next, reporting when the ray is finished.  `any`: first hit
@@ -461,6 +553,7 @@ RT_D float min3f(float a, float b, float c) {
 // scalar state stays in registers.
 struct QTrav {
     RayPre r;
+    V3 inv;
     float tmin, tmax0;
     TraceResult best;
     uint32_t node, visits, ntris;
@@ -477,6 +570,7 @@ struct QTrav {
         visits = 0;
         ntris = 0;
         sp = 0;
+        inv = V3{qinv(r.inv.x), qinv(r.inv.y), qinv(r.inv.z)};
         oct = (signbit(r.inv.x) ? 1u : 0u) | (signbit(r.inv.y) ? 2u : 0u) | (signbit(r.inv.z) ? 4u : 0u);
         any = any_hit;
     }
@@ -487,72 +581,23 @@ struct QTrav {
             dev_error(s, kDevErrIterations);
             return true;
         }
-        const uint32_t ox = oct & 1u, oy = (oct >> 1) & 1u, oz = oct >> 2;
-        const float4* np = reinterpret_cast<const float4*>(s.qnodes + node);
-        const float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3), n4 = __ldg(np + 4);
-        const uint32_t ew = __float_as_uint(n0.w);
-        const float sx = exp2_int(static_cast<int>(static_cast<int8_t>(ew & 0xffu))) * r.inv.x;
-        const float sy = exp2_int(static_cast<int>(static_cast<int8_t>((ew >> 8) & 0xffu))) * r.inv.y;
-        const float sz = exp2_int(static_cast<int>(static_cast<int8_t>((ew >> 16) & 0xffu))) * r.inv.z;
-        const float bx = (n0.x - r.org.x) * r.inv.x;
-        const float by = (n0.y - r.org.y) * r.inv.y;
-        const float bz = (n0.z - r.org.z) * r.inv.z;
-        // per axis (near, far) pairs share the scale and the offset
-        const uint64_t sx2 = pk2(sx, sx), sy2 = pk2(sy, sy), sz2 = pk2(sz, sz);
-        const uint64_t bx2 = pk2(bx, bx), by2 = pk2(by, by), bz2 = pk2(bz, bz);
-        const uint64_t m23 = pk2(-8388608.0f, -8388608.0f);
-        const float bnd = best.t;
-        uint32_t hits = 0;
-        float gmin = INFINITY;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t meta = __float_as_uint(h ? n1.w : n1.z);
-            const uint32_t lx = __float_as_uint(h ? n2.y : n2.x), hx = __float_as_uint(h ? n3.w : n3.z);
-            const uint32_t ly = __float_as_uint(h ? n2.w : n2.z), hy = __float_as_uint(h ? n4.y : n4.x);
-            const uint32_t lz = __float_as_uint(h ? n3.y : n3.x), hz = __float_as_uint(h ? n4.w : n4.z);
-            const uint32_t nx = ox ? hx : lx, fx = ox ? lx : hx;
-            const uint32_t ny = oy ? hy : ly, fy = oy ? ly : hy;
-            const uint32_t nz = oz ? hz : lz, fz = oz ? lz : hz;
-            // per byte: inner children have meta bits 4 and 3 set
-            const uint32_t inner4 = (meta & (meta << 1)) & 0x10101010u;
-            const uint32_t bit4 = (meta ^ ((inner4 >> 4) * oct)) & 0x1f1f1f1fu;
-            const uint32_t cnt4 = (meta >> 5) & 0x07070707u;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                // byte j of the near and far words as the floats 2^23 + q,
-                // minus 2^23 (exact), then t = q * s + b per plane
-                const uint32_t sel = 0x7440u + static_cast<uint32_t>(j);
-                const uint64_t qx = add2(pk2(__uint_as_float(__byte_perm(nx, 0x4B000000u, sel)),
-                                             __uint_as_float(__byte_perm(fx, 0x4B000000u, sel))), m23);
-                const uint64_t qy = add2(pk2(__uint_as_float(__byte_perm(ny, 0x4B000000u, sel)),
-                                             __uint_as_float(__byte_perm(fy, 0x4B000000u, sel))), m23);
-                const uint64_t qz = add2(pk2(__uint_as_float(__byte_perm(nz, 0x4B000000u, sel)),
-                                             __uint_as_float(__byte_perm(fz, 0x4B000000u, sel))), m23);
-                float tnx, tfx, tny, tfy, tnz, tfz;
-                upk2(fma2(qx, sx2, bx2), tnx, tfx);
-                upk2(fma2(qy, sy2, by2), tny, tfy);
-                upk2(fma2(qz, sz2, bz2), tnz, tfz);
-                const float tn = max3f(tnx, tny, fmaxf(tnz, tmin));
-                const float tf = min3f(tfx, tfy, fminf(tfz, bnd));
-                if (tn <= tf * kSlabFarScale) {
-                    const uint32_t sh = 8u * static_cast<uint32_t>(j);
-                    hits |= ((cnt4 >> sh) & 7u) << ((bit4 >> sh) & 31u);
-                    if ((inner4 >> (sh + 4u)) & 1u) gmin = fminf(gmin, tn);
-                }
-            }
+        const QNodeHits nh = qnode_test(s.qnodes + node, r.org, inv, oct, tmin, best.t);
+        // the triangles of the node's hit leaf children
+        uint32_t leaf = nh.leaf, tmask = 0;
+        while (leaf) {
+            const uint32_t m = qmeta(nh, static_cast<uint32_t>(__ffs(leaf) - 1));
+            leaf &= leaf - 1u;
+            tmask |= (m >> 5) << (m & 31u);
         }
-        // the node's leaf triangles
-        const uint32_t tbase = __float_as_uint(n1.y);
-        uint32_t tmask = hits & 0x00ffffffu;
         while (tmask) {
             const uint32_t k = static_cast<uint32_t>(__ffs(tmask) - 1);
             tmask &= tmask - 1u;
             ++ntris;
-            if (triangle(s, tbase + k)) return true;
+            if (triangle(s, nh.tri_base + k)) return true;
         }
         // next node: this node's nearest inner child, else a group from the stack
-        uint32_t gbase = __float_as_uint(n1.x), gbits = hits >> 24, gim = ew >> 24;
-        float gt = gmin;
+        uint32_t gbase = nh.child_base, gbits = nh.inner, gim = nh.imask;
+        float gt = nh.tmin;
         if (!any && gt > best.t * kSlabFarScale) gbits = 0;
         if (gbits == 0) {
             while (sp > 0) {
