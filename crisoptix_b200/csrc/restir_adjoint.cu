@@ -148,18 +148,21 @@ RT_D void mul_nee(Seg<kGrad>& sg, const BrdfGrad& g, uint32_t mi, const EmitterS
 }
 
 // Fp: TracePrefix of a valid gather prefix (path_gen.h:74-250, Conditional
-// ReSTIR), from the camera along its primary direction
+// ReSTIR), from its primary hit on.  The record holds that hit, so the
+// camera ray is not traced again (trace_closest's interaction of the stored
+// triangle and barycentrics), and the last vertex adds no factor, so the ray
+// to it is not traced at all: a prefix of the default length 2 traces none
+// of its two rays.
 template <bool kGrad>
 RT_D void seg_prefix(const RAdjView& a, const FrameParams& fp, const Prefix& cp, Seg<kGrad>& sg) {
     sg.init();
     Rng rng{cp.rng};
     const float nee = fp.p.nee_prob;
     const uint32_t max_len = static_cast<uint32_t>(fp.p.prefix_len);
-    V3 cur_pos = ld3(fp.cam.pos), cur_dir = cp.primary.dir;
-    Isect it;
-    for (uint32_t ti = 0; ti < max_len; ++ti) {
-        trace_closest(a.eval, cur_pos, cur_dir, 1e-3f, 1e16f, it);
-        if (!it.valid || ti == max_len - 1) return;
+    Isect it = unpack(a.eval, cp.primary);
+    if (it.valid) it.nrm = normalize(it.nrm);
+    for (uint32_t ti = 0; ti + 1 < max_len; ++ti) {
+        if (!it.valid) return;
         if (rng.next_float() < nee) {
             const EmitterSample es = sample_emitter(a.eval, rng);
             const V3 light_dir = normalize(es.pos - it.pos);
@@ -174,8 +177,10 @@ RT_D void seg_prefix(const RAdjView& a, const FrameParams& fp, const Prefix& cp,
         const BrdfSample bs = brdf_sample(a.samp, it, rng);
         uint32_t mi;
         sg.mul_brdf(grad_at(a, it, bs.dir, mi), mi);
-        cur_pos = it.pos;
-        cur_dir = bs.dir;
+        if (ti + 2 < max_len) {
+            const V3 pos = it.pos;
+            trace_closest(a.eval, pos, bs.dir, 1e-3f, 1e16f, it);
+        }
     }
 }
 
