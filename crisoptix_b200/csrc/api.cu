@@ -641,7 +641,7 @@ struct crisb_renderer {
     DevBuf<crisb_neighbor_rec> neighbors;
     DevBuf<uint32_t> neigh_count;
     DevBuf<float4> entries, knn_leaf;
-    DevBuf<uint32_t> pass_status, pass_flags, spatial_nbr, job_items, job_count;
+    DevBuf<uint32_t> pass_status, pass_flags, spatial_nbr, job_items;
     DevBuf<float4> shift_out, gather_state;
     DevBuf<crisb_suffix_res_rec> gather_cs;
     DevBuf<crisb_prefix_rec> gather_cp;
@@ -654,7 +654,7 @@ struct crisb_renderer {
     // machines start after them.
     DevBuf<char> machine_state;
     DevBuf<uint32_t> machine_queue[4];
-    DevBuf<uint32_t> wf_count, job_qcount;
+    DevBuf<uint32_t> counters;  // the frame's queue and list counts (Counters)
     uint32_t slots = 0;
     DevBuf<unsigned int> bounds;
     DevBuf<char> sort_temp;
@@ -714,7 +714,7 @@ struct crisb_renderer {
         b.pass_flags = pass_flags.p;
         b.spatial_nbr = spatial_nbr.p;
         b.job_items = job_items.p;
-        b.job_count = job_count.p;
+        b.job_count = nullptr;  // job_count, wf_count and job_qcount: taken by each pass
         b.shift_out = shift_out.p;
         b.gather_cs = gather_cs.p;
         b.gather_state = gather_state.p;
@@ -725,11 +725,11 @@ struct crisb_renderer {
         b.tally = timing >= 2 && ray_count.p ? ray_count.p + kRayCounters : nullptr;
         b.wf = reinterpret_cast<WfPath*>(machine_state.p);
         for (int q = 0; q < 4; ++q) b.wf_queue[q] = machine_queue[q].p;
-        b.wf_count = wf_count.p;
+        b.wf_count = nullptr;
         b.gather_cp = gather_cp.p;
         b.jobs = reinterpret_cast<ShiftJob*>(machine_state.p);
         for (int q = 0; q < 4; ++q) b.job_queue[q] = machine_queue[q].p;
-        b.job_qcount = job_qcount.p;
+        b.job_qcount = nullptr;
         return b;
     }
 
@@ -789,14 +789,10 @@ struct crisb_renderer {
         const uint32_t p = P();
         pass_status.alloc(p);
         pass_flags.alloc(p);
-        job_count.alloc(1);
         gather_cs.alloc(p);
         gather_state.alloc(2 * static_cast<size_t>(p));
         gather_cp.alloc(p);
-        wf_count.alloc(4);
-        check(cudaMemset(wf_count.p, 0, wf_count.bytes()), "memset");
-        job_qcount.alloc(4);
-        check(cudaMemset(job_qcount.p, 0, job_qcount.bytes()), "memset");
+        counters.alloc(kFrameCounters);
         allocate_jobs();
         for (int i = 0; i < 2; ++i) {
             pres[i].alloc(static_cast<size_t>(p) * (pres_bytes() / 16));
@@ -963,11 +959,12 @@ struct crisb_renderer {
         }
         Marker* m = marker();
         record(0, st);
-        launch_prefix_gen_temp_split(s, fp, bufs(), out, st, m);
-        const uint32_t sj = shift_launches_per_phase();
+        Counters cn{counters.p, st};
+        launch_prefix_gen_temp_split(s, fp, bufs(), cn, out, st, m);
         launches += params.renderer_type == CRISB_RENDERER_PATH_TRACER
                         ? 1
-                        : 2 + sj + wf_launches_per_pass(fp, 0) + prefix_pass_extra_launches(fp);
+                        : 2 + shift_launches(params, kModePrefix) + wf_launches_per_pass(fp, 0) +
+                              prefix_pass_extra_launches(fp);
         record(1, st);
         const int type = params.renderer_type;
         if (type == CRISB_RENDERER_PATH_TRACER) {
@@ -978,42 +975,46 @@ struct crisb_renderer {
         }
         if (params.prefix_enable_spatial) {
             for (int r = 0; r < params.prefix_spatial_rounds; ++r) {
-                launch_prefix_spatial(s, fp, bufs(), out, r, st, m);
+                launch_prefix_spatial(s, fp, bufs(), cn, out, r, st, m);
                 launch_prefix_copy_front_back(fp, bufs(), st);
                 if (m) m->mark(kClsOther, st);
-                launches += 3 + shift_launches_per_phase();
+                launches += 3 + shift_launches(params, kModePrefixSpatial);
             }
         }
         record(2, st);
         if (type == CRISB_RENDERER_CONDITIONAL_RESTIR) {
-            launch_suffix_gen_temp(s, fp, bufs(), st, m);
+            launch_suffix_gen_temp(s, fp, bufs(), cn, st, m);
             scur ^= 1;
-            launches += 2 + sj + wf_launches_per_pass(fp, 1);
+            launches += 2 + shift_launches(params, kModeTemporal) + wf_launches_per_pass(fp, 1);
             record(3, st);
             if (params.suffix_enable_spatial && params.suffix_spatial_count > 0) {
                 for (int r = 0; r < params.suffix_spatial_rounds; ++r) {
-                    launch_suffix_spatial(s, fp, bufs(), st, m);
-                    launches += 2 + sj;
+                    launch_suffix_spatial(s, fp, bufs(), cn, st, m);
+                    launches += 2 + shift_launches(params, kModeSpatial);
                     scur ^= 1;
                 }
             }
             record(4, st);
-            lbvh::Work w = knn.work(err.p);
-            launch_store_entries(s, fp, bufs(), w, bounds.p, st);
-            check(rsort::sort_high32(knn.keys_in.p, knn.keys.p, sort_temp.p, sort_temp.bytes(), P(), st),
-                  "radix sort");
-            launch_knn_finish(fp, bufs(), w, knn_leaf.p, st);
-            if (m) m->mark(kClsSearch, st);
-            launches += 3 + 4 + rsort::kLaunches;
+            // without gather neighbours nothing queries the endpoint structure
+            if (K() > 0) {
+                lbvh::Work w = knn.work(err.p);
+                launch_store_entries(s, fp, bufs(), w, bounds.p, st);
+                check(rsort::sort_high32(knn.keys_in.p, knn.keys.p, sort_temp.p, sort_temp.bytes(), P(), st),
+                      "radix sort");
+                launch_knn_finish(fp, bufs(), w, knn_leaf.p, st);
+                if (m) m->mark(kClsSearch, st);
+                launches += 3 + 4 + rsort::kLaunches;
+            }
             record(5, st);
             if (params.gather_n > 1 && !gather_ext.p) {
                 gather_ext.alloc(3 * static_cast<size_t>(P()));
                 gather_last.alloc(P());
             }
-            launch_final_gather_split(s, fp, bufs(), out, st, m);
-            launches += 3 + sj + wf_launches_per_pass(fp, 2);
+            launch_final_gather_split(s, fp, bufs(), cn, out, st, m);
+            launches += 1 + wf_launches_per_pass(fp, 2);
+            if (K() > 0) launches += 2 + shift_launches(params, kModeGather);
             if (params.gather_n > 1)
-                launches += 1 + static_cast<uint32_t>(params.gather_n - 1) * (3 + sj);
+                launches += 1 + static_cast<uint32_t>(params.gather_n - 1) * (3 + shift_launches(params, kModeGatherExtra));
         } else {
             record(3, st);
             record(4, st);

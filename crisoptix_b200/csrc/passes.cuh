@@ -71,7 +71,7 @@ struct Bufs {
     uint32_t* pass_flags;   // P
     uint32_t* spatial_nbr;  // P * slots / 2
     uint32_t* job_items;    // P * slots
-    uint32_t* job_count;    // 1
+    uint32_t* job_count;    // 1, of the phase (Counters)
     float4* shift_out;      // P * slots: shifted f (xyz) and Jacobian (w)
     crisb_suffix_res_rec* gather_cs;  // P: canonical suffix of the final gather
     // gatherN > 1 only (else null): per pixel the camera ray direction (xyz, w
@@ -88,16 +88,16 @@ struct Bufs {
     // resampling kernel for the work present in the frame (kTally*)
     unsigned long long* tally;
     // wavefront path tracing: one path state per pixel, ray queues of two
-    // rounds (closest, shadow) x 2 and their counts
+    // rounds (closest, shadow) x 2 and the counts of every round of the pass
     WfPath* wf;
     uint32_t* wf_queue[4];
-    uint32_t* wf_count;          // 4
+    uint32_t* wf_count;          // 2 per round (Counters)
     crisb_prefix_rec* gather_cp; // canonical prefix of the final gather
     // shift machines: one record per job of the list, ray queues of two
-    // rounds (closest, shadow) x 2 and their counts
+    // rounds (closest, shadow) x 2 and the counts of every round of the phase
     ShiftJob* jobs;         // P * slots
     uint32_t* job_queue[4]; // P * slots each
-    uint32_t* job_qcount;   // 4
+    uint32_t* job_qcount;   // 2 per round (Counters)
 
     RT_HD KnnView knn() const { return KnnView{knn_nodes, knn_leaf, knn_pixel, knn_n}; }
 };
@@ -127,24 +127,63 @@ constexpr int kTriLeafMax = 4;
 // binary levels of SAH splits before the scene builder switches to median splits
 constexpr int kMedianDepth = 40;
 
-void launch_prefix_spatial(const SceneView& s, const FrameParams& fp, const Bufs& b, float* out, int round,
+// Queue and list counters of a frame: each pass takes cleared ones from one
+// array, which a memset on the frame's stream clears at the frame's start and
+// whenever it runs out (a pass takes all of its counters at once, so those
+// given out before are done with in stream order).  Clearing two counters
+// before every round instead cost a memset node of its own each time: 31 of
+// the 132 nodes of a 256 x 256 Cornell frame, 2-3 us apiece with their gaps.
+constexpr uint32_t kFrameCounters = 4096;
+struct Counters {
+    uint32_t* p;
+    cudaStream_t st;
+    uint32_t used = kFrameCounters;
+    uint32_t* take(uint32_t n) {
+        if (n > kFrameCounters - used) {
+            cudaMemsetAsync(p, 0, kFrameCounters * sizeof(uint32_t), st);
+            used = 0;
+        }
+        uint32_t* r = p + used;
+        used += n;
+        return r;
+    }
+};
+
+void launch_prefix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out, int round,
                            cudaStream_t st, Marker* m);
 void launch_prefix_copy_front_back(const FrameParams& fp, const Bufs& b, cudaStream_t st);
 // reuse passes as per-pixel kernel -> compacted shift jobs -> per-pixel combine
-void launch_prefix_gen_temp_split(const SceneView& s, const FrameParams& fp, const Bufs& b, float* out,
+void launch_prefix_gen_temp_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                   cudaStream_t st, Marker* m);
-void launch_suffix_gen_temp(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
-void launch_suffix_spatial(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
-void launch_final_gather_split(const SceneView& s, const FrameParams& fp, const Bufs& b, float* out,
+void launch_suffix_gen_temp(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, cudaStream_t st,
+                            Marker* m);
+void launch_suffix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, cudaStream_t st,
+                           Marker* m);
+void launch_final_gather_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                cudaStream_t st, Marker* m);
-// wavefront path tracing (wavefront.cu): init + rounds of trace / shade
+// wavefront path tracing (wavefront.cu): init + rounds of trace / shade;
+// b.wf_count holds 2 x wf_round_count cleared counters
+int wf_round_count(const crisb_params& p, int flow);
 void launch_wf_prefix(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
 void launch_wf_suffix(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
 void launch_wf_gather(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
 // kernels of one wavefront pass of `flow` (0 prefix, 1 suffix, 2 gather)
 uint32_t wf_launches_per_pass(const FrameParams& fp, int flow);
 // kernels of one shift-job phase (begin + rounds of closest / shadow / step)
-uint32_t shift_launches_per_phase();
+uint32_t shift_launches(const crisb_params& p, int mode);
+// what a shift phase shifts (the job's source and destination)
+enum ShiftMode : int {
+    kModeTemporal = 0,  // suffix temporal reuse
+    kModeSpatial = 1,   // suffix spatial reuse
+    kModeGather = 2,    // final gather
+    kModePrefix = 3,    // prefix temporal reuse (slot 0: previous onto canonical)
+    // prefix spatial reuse (slot 2n: neighbour n onto the pixel's prefix; 2n + 1:
+    // the pixel's prefix onto neighbour n's)
+    kModePrefixSpatial = 4,
+    // the final gather's extra prefixes (slot 2n: neighbour n's suffix onto the
+    // extra prefix's last vertex)
+    kModeGatherExtra = 5,
+};
 // kernels the prefix pass adds after its combine (the reprojection back copy)
 uint32_t prefix_pass_extra_launches(const FrameParams& fp);
 // prefix entries, endpoint bounds/count and Morton keys (w.keys_in); the

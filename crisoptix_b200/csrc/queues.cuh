@@ -135,26 +135,32 @@ unsigned trace_grid_of() {
     return g;
 }
 
-template <class R, int kFmt>
-void launch_trace_fmt(uint32_t block, uint32_t m, cudaStream_t st, const SceneView& s, const uint32_t* qc,
-                      const uint32_t* ccnt, const uint32_t* qs, const uint32_t* scnt, R* rec) {
-    if (block == 64)
-        k_q_trace<R, 64, kFmt><<<trace_grid_of<R, 64, kFmt>() * m, 64, 0, st>>>(s, qc, ccnt, qs, scnt, rec);
-    else if (block == 256)
-        k_q_trace<R, 256, kFmt><<<trace_grid_of<R, 256, kFmt>() * m, 256, 0, st>>>(s, qc, ccnt, qs, scnt, rec);
-    else
-        k_q_trace<R, 128, kFmt><<<trace_grid_of<R, 128, kFmt>() * m, 128, 0, st>>>(s, qc, ccnt, qs, scnt, rec);
+template <class R, int kB, int kFmt>
+void launch_trace_as(uint32_t m, uint32_t most, cudaStream_t st, const SceneView& s, const uint32_t* qc,
+                     const uint32_t* ccnt, const uint32_t* qs, const uint32_t* scnt, R* rec) {
+    const unsigned g = std::min(trace_grid_of<R, kB, kFmt>() * m, std::max(most, 1u) / kB + 1);
+    k_q_trace<R, kB, kFmt><<<g, kB, 0, st>>>(s, qc, ccnt, qs, scnt, rec);
 }
 
-// one traversal launch over a closest-hit and a shadow queue: `block`
-// threads (64, 128 or 256) and `mult` x the blocks resident at once, the
-// kernel instance of the scene tree's node format
+template <class R, int kFmt>
+void launch_trace_fmt(uint32_t block, uint32_t m, uint32_t most, cudaStream_t st, const SceneView& s,
+                      const uint32_t* qc, const uint32_t* ccnt, const uint32_t* qs, const uint32_t* scnt, R* rec) {
+    if (block == 64) launch_trace_as<R, 64, kFmt>(m, most, st, s, qc, ccnt, qs, scnt, rec);
+    else if (block == 256) launch_trace_as<R, 256, kFmt>(m, most, st, s, qc, ccnt, qs, scnt, rec);
+    else launch_trace_as<R, 128, kFmt>(m, most, st, s, qc, ccnt, qs, scnt, rec);
+}
+
+// one traversal launch over a closest-hit and a shadow queue that hold at most
+// `most` rays together: `block` threads (64, 128 or 256) and `mult` x the blocks
+// resident at once, but no more than the rays fill (a 256 x 256 frame: 513
+// instead of 9,472 blocks a launch, 343 -> 341 us); the kernel instance of the
+// scene tree's node format
 template <class R>
-void launch_trace(uint32_t block, uint32_t mult, cudaStream_t st, const SceneView& s, const uint32_t* qc,
-                  const uint32_t* ccnt, const uint32_t* qs, const uint32_t* scnt, R* rec) {
+void launch_trace(uint32_t block, uint32_t mult, uint32_t most, cudaStream_t st, const SceneView& s,
+                  const uint32_t* qc, const uint32_t* ccnt, const uint32_t* qs, const uint32_t* scnt, R* rec) {
     const uint32_t m = std::max(mult, 1u);
-    if (s.qnodes) launch_trace_fmt<R, kFmtCompressed8>(block, m, st, s, qc, ccnt, qs, scnt, rec);
-    else launch_trace_fmt<R, kFmtWide4>(block, m, st, s, qc, ccnt, qs, scnt, rec);
+    if (s.qnodes) launch_trace_fmt<R, kFmtCompressed8>(block, m, most, st, s, qc, ccnt, qs, scnt, rec);
+    else launch_trace_fmt<R, kFmtWide4>(block, m, most, st, s, qc, ccnt, qs, scnt, rec);
 }
 
 }  // namespace

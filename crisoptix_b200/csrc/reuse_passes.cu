@@ -28,8 +28,6 @@ constexpr uint32_t kStFinal = 0;      // nothing left to do in the combine kerne
 constexpr uint32_t kStCanonOnly = 1;  // temporal: stream the canonical sample only
 constexpr uint32_t kStReuse = 2;      // reuse with the shift results
 
-enum ShiftMode : int { kModeTemporal = 0, kModeSpatial = 1, kModeGather = 2 };
-
 constexpr uint32_t kSlotBits = 6;  // job code = pixel << 6 | slot
 
 // Append the job slots set in `mask` for pixel i to the list.  Every thread of
@@ -85,14 +83,6 @@ RT_D void count_jobs(const SceneView& s, uint32_t total) {
 // / 1.20 ms per 1080p frame but added more in traversal launches (frame 17.04
 // -> 17.20 / 17.32 / 17.35 ms).
 constexpr int kShiftRounds = 3;
-constexpr int kModePrefix = 3;  // prefix temporal reuse (slot 0: previous onto canonical)
-// prefix spatial reuse (slot 2n: neighbour n onto the pixel's prefix; 2n + 1:
-// the pixel's prefix onto neighbour n's)
-constexpr int kModePrefixSpatial = 4;
-// the final gather's extra prefixes (slot 2n: neighbour n's suffix onto the
-// extra prefix's last vertex)
-constexpr int kModeGatherExtra = 5;
-
 RT_HD bool prefix_mode(int mode) { return mode == kModePrefix || mode == kModePrefixSpatial; }
 
 // source path of a job
@@ -258,9 +248,11 @@ RT_D void job_store(ShiftJob* r, const ShiftJob& j) {
     r->ctr = j.ctr;
 }
 
+// queue job t's ray for round `round` (two queue pairs, used in turn)
 RT_D void job_push(const Bufs& b, int round, int req, uint32_t t) {
-    q_append(b.job_queue[2 * round], &b.job_qcount[2 * round], req == kReqClosest, t);
-    q_append(b.job_queue[2 * round + 1], &b.job_qcount[2 * round + 1], req == kReqShadow, t);
+    const int q = 2 * (round & 1);
+    q_append(b.job_queue[q], &b.job_qcount[2 * round], req == kReqClosest, t);
+    q_append(b.job_queue[q + 1], &b.job_qcount[2 * round + 1], req == kReqShadow, t);
 }
 
 // first step of every job of the list: the checks of the reference function,
@@ -326,14 +318,14 @@ __global__ void __launch_bounds__(kPassBlock) k_shift_overflow(SceneView s, Fram
     }
 }
 
-// resume every job whose ray of round `cur` finished; in the last round jobs
+// resume every job whose ray of round `round` finished; in the last round jobs
 // with replays left finish inline
 template <bool kLast, bool kTex>
-__global__ void __launch_bounds__(kPassBlock) k_shift_step(SceneView s, FrameParams fp, Bufs b, int mode, int cur) {
-    const uint32_t nc = b.job_qcount[2 * cur], ns = b.job_qcount[2 * cur + 1];
+__global__ void __launch_bounds__(kPassBlock) k_shift_step(SceneView s, FrameParams fp, Bufs b, int mode, int round) {
+    const uint32_t nc = b.job_qcount[2 * round], ns = b.job_qcount[2 * round + 1];
     const uint32_t total = nc + ns;
-    const uint32_t* qc = b.job_queue[2 * cur];
-    const uint32_t* qs = b.job_queue[2 * cur + 1];
+    const uint32_t* qc = b.job_queue[2 * (round & 1)];
+    const uint32_t* qs = b.job_queue[2 * (round & 1) + 1];
     const bool prefix = prefix_mode(mode);
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (uint32_t base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
@@ -375,7 +367,7 @@ __global__ void __launch_bounds__(kPassBlock) k_shift_step(SceneView s, FramePar
                 }
             }
         }
-        if (!kLast) job_push(b, cur ^ 1, req, t);
+        if (!kLast) job_push(b, round + 1, req, t);
     }
 }
 
@@ -622,6 +614,7 @@ __global__ void __launch_bounds__(kPassBlock) k_gather_finish(FrameParams fp, Bu
     if (i >= pixel_count(fp)) return;
     uint32_t st = kStFinal;
     V3 direct = splat(0.0f);
+    if (fp.k == 0) b.neigh_count[i] = 0;  // no query runs
     if (b.pass_status[i] == kWfPath) {
         b.gbuf[i].rng = b.wf[i].rng;
         const Prefix cp = ld_prefix_v(b.gather_cp[i]);
@@ -1124,26 +1117,45 @@ const ShiftGrids& shift_grids() {
         if (m) m->mark(cls, st); \
     } while (0)
 
+// Rounds of a shift phase: at most kShiftRounds, fewer where the jobs trace
+// fewer rays.  A prefix shift replays the vertices before its reconnection
+// vertex but the first two (none for a prefix of length 2) and then tests the
+// edge.  At least one: a reservoir kept from a frame with another prefix length
+// may need more rays, which the last round's step traces in place.
+int shift_rounds(const crisb_params& p, int mode) {
+    if (!prefix_mode(mode)) return kShiftRounds;
+    const int len = p.renderer_type == CRISB_RENDERER_CONDITIONAL_RESTIR ? p.prefix_len : p.max_path_len;
+    return std::min(std::max(len - 1, 1), kShiftRounds);
+}
+
+// the counters of one shift phase and, with `rounds` > 0, a wavefront pass
+void take_counters(Bufs& b, Counters& c, int rounds) {
+    // max_path_len <= 255 keeps a pass well below the array's size
+    uint32_t* p = c.take(2 * static_cast<uint32_t>(rounds) + 1 + 2 * kShiftRounds);
+    b.wf_count = p;
+    b.job_count = p + 2 * rounds;
+    b.job_qcount = b.job_count + 1;
+}
+
 // the shift jobs of the list: begin, then rounds of trace / step
 template <bool kTex>
 void run_shift_jobs_as(const SceneView& s, const FrameParams& fp, const Bufs& b, int mode, cudaStream_t st,
                        Marker* m) {
     const ShiftGrids& g = shift_grids<kTex>();
-    cudaMemsetAsync(b.job_qcount, 0, 2 * sizeof(uint32_t), st);
+    const int rounds = shift_rounds(fp.p, mode);
     k_shift_begin<kTex><<<g.begin, kPassBlock, 0, st>>>(s, fp, b, mode);
     MARK(kClsShift);
     k_shift_overflow<kTex><<<g.overflow, kPassBlock, 0, st>>>(s, fp, b, mode);
     MARK(kClsShift);
-    for (int r = 0; r < kShiftRounds; ++r) {
-        const int cur = r & 1, nxt = cur ^ 1;
-        launch_trace<ShiftJob>(fp.trace_block, fp.trace_grid, st, s, b.job_queue[2 * cur], b.job_qcount + 2 * cur,
-                               b.job_queue[2 * cur + 1], b.job_qcount + 2 * cur + 1, b.jobs);
+    for (int r = 0; r < rounds; ++r) {
+        const int q = 2 * (r & 1);
+        launch_trace<ShiftJob>(fp.trace_block, fp.trace_grid, b.job_cap, st, s, b.job_queue[q], b.job_qcount + 2 * r,
+                               b.job_queue[q + 1], b.job_qcount + 2 * r + 1, b.jobs);
         MARK(kClsTrace);
-        if (r + 1 < kShiftRounds) {
-            cudaMemsetAsync(b.job_qcount + 2 * nxt, 0, 2 * sizeof(uint32_t), st);
-            k_shift_step<false, kTex><<<g.step, kPassBlock, 0, st>>>(s, fp, b, mode, cur);
+        if (r + 1 < rounds) {
+            k_shift_step<false, kTex><<<g.step, kPassBlock, 0, st>>>(s, fp, b, mode, r);
         } else {
-            k_shift_step<true, kTex><<<g.step_last, kPassBlock, 0, st>>>(s, fp, b, mode, cur);
+            k_shift_step<true, kTex><<<g.step_last, kPassBlock, 0, st>>>(s, fp, b, mode, r);
         }
         MARK(kClsShift);
     }
@@ -1162,17 +1174,19 @@ void run_shift_jobs(const SceneView& s0, const FrameParams& fp, const Bufs& b, i
 
 }  // namespace
 
-uint32_t shift_launches_per_phase() { return 2 + 2 * kShiftRounds; }
+uint32_t shift_launches(const crisb_params& p, int mode) {
+    return 2 + 2 * static_cast<uint32_t>(shift_rounds(p, mode));
+}
 
-void launch_prefix_gen_temp_split(const SceneView& s, const FrameParams& fp, const Bufs& b, float* out,
+void launch_prefix_gen_temp_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                   cudaStream_t st, Marker* m) {
     if (fp.p.renderer_type == CRISB_RENDERER_PATH_TRACER) {
         k_path_tracer<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, out);
         MARK(kClsOther);
         return;
     }
+    take_counters(b, c, wf_round_count(fp.p, 0));
     launch_wf_prefix(s, fp, b, st, m);
-    cudaMemsetAsync(b.job_count, 0, sizeof(uint32_t), st);
     k_prefix_finish<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b, out);
     MARK(kClsShade);
     run_shift_jobs(s, fp, b, kModePrefix, st, m);
@@ -1188,9 +1202,9 @@ uint32_t prefix_pass_extra_launches(const FrameParams& fp) {
     return prefix_back_copy(fp) && fp.p.motion_mode != CRISB_MOTION_NONE ? 1u : 0u;
 }
 
-void launch_prefix_spatial(const SceneView& s, const FrameParams& fp, const Bufs& b, float* out, int round,
+void launch_prefix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out, int round,
                            cudaStream_t st, Marker* m) {
-    cudaMemsetAsync(b.job_count, 0, sizeof(uint32_t), st);
+    take_counters(b, c, 0);
     k_prefix_spatial_select<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     MARK(kClsResample);
     run_shift_jobs(s, fp, b, kModePrefixSpatial, st, m);
@@ -1198,9 +1212,10 @@ void launch_prefix_spatial(const SceneView& s, const FrameParams& fp, const Bufs
     MARK(kClsResample);
 }
 
-void launch_suffix_gen_temp(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m) {
+void launch_suffix_gen_temp(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, cudaStream_t st,
+                            Marker* m) {
+    take_counters(b, c, wf_round_count(fp.p, 1));
     launch_wf_suffix(s, fp, b, st, m);
-    cudaMemsetAsync(b.job_count, 0, sizeof(uint32_t), st);
     k_suffix_temp_finish<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     MARK(kClsShade);
     run_shift_jobs(s, fp, b, kModeTemporal, st, m);
@@ -1208,8 +1223,9 @@ void launch_suffix_gen_temp(const SceneView& s, const FrameParams& fp, const Buf
     MARK(kClsResample);
 }
 
-void launch_suffix_spatial(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m) {
-    cudaMemsetAsync(b.job_count, 0, sizeof(uint32_t), st);
+void launch_suffix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, cudaStream_t st,
+                           Marker* m) {
+    take_counters(b, c, 0);
     k_suffix_spatial_select<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     MARK(kClsResample);
     run_shift_jobs(s, fp, b, kModeSpatial, st, m);
@@ -1217,20 +1233,22 @@ void launch_suffix_spatial(const SceneView& s, const FrameParams& fp, const Bufs
     MARK(kClsResample);
 }
 
-void launch_final_gather_split(const SceneView& s, const FrameParams& fp, const Bufs& b, float* out,
+void launch_final_gather_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                cudaStream_t st, Marker* m) {
+    take_counters(b, c, wf_round_count(fp.p, 2));
     launch_wf_gather(s, fp, b, st, m);
     k_gather_finish<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b, out);
     MARK(kClsShade);
-    cudaMemsetAsync(b.job_count, 0, sizeof(uint32_t), st);
-    k_gather_query<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b);
-    MARK(kClsSearch);
-    run_shift_jobs(s, fp, b, kModeGather, st, m);
-    k_gather_combine<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b, out);
-    MARK(kClsResample);
+    if (fp.k > 0) {  // without neighbours k_gather_finish has stored every pixel's result
+        k_gather_query<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b);
+        MARK(kClsSearch);
+        run_shift_jobs(s, fp, b, kModeGather, st, m);
+        k_gather_combine<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b, out);
+        MARK(kClsResample);
+    }
     if (fp.p.gather_n > 1) {
         for (int g = 1; g < fp.p.gather_n; ++g) {
-            cudaMemsetAsync(b.job_count, 0, sizeof(uint32_t), st);
+            take_counters(b, c, 0);
             k_gather_extra_prefix<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b);
             MARK(kClsShade);
             k_gather_extra_query<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b);

@@ -22,9 +22,11 @@ namespace crisb {
 
 namespace {
 
+// queue path i's ray for round `round` (two queue pairs, used in turn)
 RT_D void wf_push(const Bufs& b, int round, int req, uint32_t i) {
-    q_append(b.wf_queue[2 * round], &b.wf_count[2 * round], req == kReqClosest, i);
-    q_append(b.wf_queue[2 * round + 1], &b.wf_count[2 * round + 1], req == kReqShadow, i);
+    const int q = 2 * (round & 1);
+    q_append(b.wf_queue[q], &b.wf_count[2 * round], req == kReqClosest, i);
+    q_append(b.wf_queue[q + 1], &b.wf_count[2 * round + 1], req == kReqShadow, i);
 }
 
 RT_D WfPath wf_blank() {
@@ -265,7 +267,7 @@ __global__ void __launch_bounds__(kPassBlock) k_wf_init_gather(FrameParams fp, B
     wf_push(b, 0, req, i);
 }
 
-// ---- shading: resume every path whose ray of round `cur` finished ---------------------
+// ---- shading: resume every path whose ray of round `round` finished ---------------------
 template <bool kTex>
 RT_D int wf_step(const SceneView& s, const FrameParams& fp, const Bufs& b, int flow, uint32_t i, WfPath& w,
                  Rng& rng) {
@@ -309,8 +311,8 @@ RT_D void wf_trace_inline(const SceneView& s, WfPath& w, int req) {
     }
 }
 
-// Resume every path whose ray of round `cur` finished and queue its next ray;
-// with kInline (the last wavefront round) trace the path's remaining rays in
+// Resume every path whose ray of round `round` finished and queue its next ray;
+// with kInline (the suffix flow's last round) trace the path's remaining rays in
 // place until it ends, so the few long paths left do not cost a trace and a
 // shade launch per bounce.  One launch over both queues: a separate instance
 // for the shadow-ray results (94 against 126 registers) cost more in launches
@@ -319,12 +321,11 @@ RT_D void wf_trace_inline(const SceneView& s, WfPath& w, int req) {
 // at 5 resident blocks per SM (96 registers; shading 3.86 -> 3.78 ms per
 // 1080p frame against one kernel for both), the textured one at 4.
 template <bool kInline, bool kTex>
-__global__ void __launch_bounds__(kPassBlock, kInline ? 1 : (kTex ? 4 : 5)) k_wf_shade(SceneView s, FrameParams fp, Bufs b, int flow, int cur) {
-    const uint32_t nc = b.wf_count[2 * cur], ns = b.wf_count[2 * cur + 1];
+__global__ void __launch_bounds__(kPassBlock, kInline ? 1 : (kTex ? 4 : 5)) k_wf_shade(SceneView s, FrameParams fp, Bufs b, int flow, int round, int rounds) {
+    const uint32_t nc = b.wf_count[2 * round], ns = b.wf_count[2 * round + 1];
     const uint32_t total = nc + ns;
-    const uint32_t* qc = b.wf_queue[2 * cur];
-    const uint32_t* qs = b.wf_queue[2 * cur + 1];
-    const int nxt = cur ^ 1;
+    const uint32_t* qc = b.wf_queue[2 * (round & 1)];
+    const uint32_t* qs = b.wf_queue[2 * (round & 1) + 1];
     // a path traces at most a prefix, a suffix and one shadow ray per vertex
     const int max_steps = 4 * (fp.p.max_path_len + 2);
     for (uint32_t base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
@@ -350,7 +351,10 @@ __global__ void __launch_bounds__(kPassBlock, kInline ? 1 : (kTex ? 4 : 5)) k_wf
             w.rng = rng.state;
             wf_store(b.wf, i, w);
         }
-        if (!kInline) wf_push(b, nxt, req, i);
+        if (!kInline) {
+            if (round + 1 < rounds) wf_push(b, round + 1, req, i);
+            else if (req != kReqDone) dev_error(s, kDevErrIterations);
+        }
     }
 }
 
@@ -369,34 +373,21 @@ const WfGrids& wf_grids() {
     return g;
 }
 
-// Wavefront rounds of a pass: a path traces at most max_path_len + 1 rays
-// after its first; the shading kernel of the last round finishes any path
-// still running in place.  Finishing in place from an earlier round (3 to 6)
-// saved traversal launches but cost as much in the in-place kernel on the
-// 1080p workload (24.2 ms/frame either way).
-// (the ConditionalRestir prefix flow stops after prefix_len vertices: at most
-// prefix_len closest-hit rays and one shadow ray per path)
-int wf_round_count(const FrameParams& fp, int flow) {
-    if (flow == 0 && fp.p.renderer_type == CRISB_RENDERER_CONDITIONAL_RESTIR)
-        return std::min(fp.p.prefix_len + 2, fp.p.max_path_len + 2);
-    return fp.p.max_path_len + 2;
-}
-
 // rounds after the init kernel
 template <bool kTex>
 void wf_rounds_t(const SceneView& s, const FrameParams& fp, const Bufs& b, int flow, cudaStream_t st, Marker* m) {
     const WfGrids& g = wf_grids<kTex>();
-    const int rounds = wf_round_count(fp, flow);
+    const int rounds = wf_round_count(fp.p, flow);
+    const unsigned most = grid_for(fp.width * fp.height);  // a path a pixel
     for (int r = 0; r < rounds; ++r) {
-        const int cur = r & 1, nxt = cur ^ 1;
-        launch_trace<WfPath>(fp.trace_block, fp.trace_grid, st, s, b.wf_queue[2 * cur], b.wf_count + 2 * cur,
-                             b.wf_queue[2 * cur + 1], b.wf_count + 2 * cur + 1, b.wf);
+        const int q = 2 * (r & 1);
+        launch_trace<WfPath>(fp.trace_block, fp.trace_grid, fp.width * fp.height, st, s, b.wf_queue[q],
+                             b.wf_count + 2 * r, b.wf_queue[q + 1], b.wf_count + 2 * r + 1, b.wf);
         if (m) m->mark(kClsTrace, st);
-        if (r + 1 < rounds) {
-            cudaMemsetAsync(b.wf_count + 2 * nxt, 0, 2 * sizeof(uint32_t), st);
-            k_wf_shade<false, kTex><<<g.shade, kPassBlock, 0, st>>>(s, fp, b, flow, cur);
+        if (r + 1 < rounds || flow != 1) {
+            k_wf_shade<false, kTex><<<std::min(g.shade, most), kPassBlock, 0, st>>>(s, fp, b, flow, r, rounds);
         } else {
-            k_wf_shade<true, kTex><<<g.shade_inline, kPassBlock, 0, st>>>(s, fp, b, flow, cur);
+            k_wf_shade<true, kTex><<<std::min(g.shade_inline, most), kPassBlock, 0, st>>>(s, fp, b, flow, r, rounds);
         }
         if (m) m->mark(kClsShade, st);
     }
@@ -409,12 +400,30 @@ void wf_rounds(const SceneView& s, const FrameParams& fp, const Bufs& b, int flo
 
 }  // namespace
 
+// Wavefront rounds of a pass: the most rays a path of the flow traces.  (A
+// suffix may continue a prefix that temporal reuse kept from a frame with another
+// prefix length, and so be longer: the suffix flow's last shading kernel
+// finishes paths still running in place.)  A ConditionalRestir prefix stops after prefix_len vertices, or at
+// an earlier one with a shadow ray: prefix_len rays.  Its suffix has
+// n = max_path_len - prefix_len vertices, the first of them known: n - 1 rays to
+// the others, the shadow ray and the reconnection-vertex ray of the last.  The
+// gather traces one after the other.  A RestirPt prefix: max_path_len vertices
+// and a shadow ray.  (Finishing in place from an earlier round, 3 to 6, saved
+// traversal launches but cost as much in the in-place kernel on the 1080p
+// workload, 24.2 ms/frame either way; the two to three empty rounds of
+// max_path_len + 2 for every flow cost 14 us each.)
+int wf_round_count(const crisb_params& p, int flow) {
+    if (p.renderer_type != CRISB_RENDERER_CONDITIONAL_RESTIR) return p.max_path_len + 1;
+    const int suffix = p.max_path_len > p.prefix_len ? p.max_path_len - p.prefix_len + 1 : 0;
+    const int rays = (flow != 1 ? p.prefix_len : 0) + (flow != 0 ? suffix : 0);
+    return std::max(rays, 1);
+}
+
 uint32_t wf_launches_per_pass(const FrameParams& fp, int flow) {
-    return 1 + 2 * static_cast<uint32_t>(wf_round_count(fp, flow));
+    return 1 + 2 * static_cast<uint32_t>(wf_round_count(fp.p, flow));
 }
 
 void launch_wf_prefix(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m) {
-    cudaMemsetAsync(b.wf_count, 0, 2 * sizeof(uint32_t), st);
     if (fp.shared_stage) k_wf_init_prefix<true><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     else k_wf_init_prefix<false><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     if (m) m->mark(kClsShade, st);
@@ -422,7 +431,6 @@ void launch_wf_prefix(const SceneView& s, const FrameParams& fp, const Bufs& b, 
 }
 
 void launch_wf_suffix(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m) {
-    cudaMemsetAsync(b.wf_count, 0, 2 * sizeof(uint32_t), st);
     if (s.mat_tex) k_wf_init_suffix<true><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b);
     else k_wf_init_suffix<false><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b);
     if (m) m->mark(kClsShade, st);
@@ -430,7 +438,6 @@ void launch_wf_suffix(const SceneView& s, const FrameParams& fp, const Bufs& b, 
 }
 
 void launch_wf_gather(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m) {
-    cudaMemsetAsync(b.wf_count, 0, 2 * sizeof(uint32_t), st);
     if (fp.shared_stage) k_wf_init_gather<true><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     else k_wf_init_gather<false><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     if (m) m->mark(kClsShade, st);
