@@ -969,15 +969,43 @@ RT_D void prefix_tail(const FrameParams& fp, const Bufs& b, float* out, uint32_t
     if (prefix_back_copy(fp) && fp.p.motion_mode == CRISB_MOTION_NONE) st_pres(b.pres[fp.back], i, cur);
 }
 
-// PathTracer mode: TraceCompletePath per pixel (prefix_gen_temp_reuse.cu:175-192)
-__global__ void __launch_bounds__(kPassBlock) k_path_tracer(SceneView s, FrameParams fp, float* out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= pixel_count(fp)) return;
-    Rng rng = rng_seeded(tea64(i, fp.random));
-    const V3 dir = camera_dir(fp, i % fp.width, i / fp.width, rng);
-    V3 L = trace_complete_path(s, fp, ld3(fp.cam.pos), dir, rng);
-    if (nonfinite(L)) L = splat(0.0f);
-    store_output(fp, out, i, L);
+// PathTracer mode: TraceCompletePath per pixel (prefix_gen_temp_reuse.cu:175-192).
+// Persistent warps whose lanes take the next pixel as their paths end, one ray of
+// either kind per lane and turn: 1.87 -> 1.15 ms for a 960x540 frame of the large
+// scene against a thread a pixel (2.0 G rays/s).  4 / 5 / 6 / 7 resident blocks
+// (115, 94, 80, 72 registers): 1.25 / 1.15 / 1.13 / 1.19 ms; refilling only once 8 or
+// 16 lanes are idle: 1.15 / 1.23 ms.
+template <bool kTex>
+__global__ void __launch_bounds__(kPassBlock, 5) k_path_tracer(SceneView s, FrameParams fp, float* out) {
+    PixelPool pool(pixel_count(fp));
+    CompletePath path;
+    uint32_t pixel = 0xffffffffu;
+    while (true) {
+        const unsigned idle = __ballot_sync(0xffffffffu, pixel == 0xffffffffu);
+        if (idle) {
+            const bool more = pool.more();
+            if (idle == 0xffffffffu && !more) break;
+            if (more) {
+                const uint32_t i = pool.take(pixel == 0xffffffffu);
+                if (i != 0xffffffffu) {
+                    pixel = i;
+                    Rng rng = rng_seeded(tea64(i, fp.random));
+                    const V3 dir = camera_dir(fp, i % fp.width, i / fp.width, rng);
+                    path.begin(ld3(fp.cam.pos), dir, rng);
+                }
+            }
+        }
+        if (pixel != 0xffffffffu) {
+            count_ray(s, path.shadow ? 1 : 0);
+            const TraceResult h = traverse_ray(s, path.o, path.d, 1e-3f, path.tmax, path.shadow);
+            if (!path.template step<kTex>(s, fp, h)) {
+                V3 L = path.radiance;
+                if (nonfinite(L)) L = splat(0.0f);
+                store_output(fp, out, pixel, L);
+                pixel = 0xffffffffu;
+            }
+        }
+    }
 }
 
 // per pixel after the canonical prefixes (wavefront.cu, prefix flow) finished:
@@ -1094,6 +1122,12 @@ __global__ void __launch_bounds__(kPassBlock, kResampleMinBlocks) k_prefix_combi
     prefix_tail(fp, b, out, i, cur, true);
 }
 
+template <bool kTex>
+unsigned path_tracer_grid() {
+    static const unsigned g = persistent_grid(reinterpret_cast<const void*>(k_path_tracer<kTex>));
+    return g;
+}
+
 struct ShiftGrids {
     unsigned begin, step, step_last, overflow;
 };
@@ -1181,7 +1215,9 @@ uint32_t shift_launches(const crisb_params& p, int mode) {
 void launch_prefix_gen_temp_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                   cudaStream_t st, Marker* m) {
     if (fp.p.renderer_type == CRISB_RENDERER_PATH_TRACER) {
-        k_path_tracer<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, out);
+        const unsigned most = grid_for(fp.width * fp.height);
+        if (s.mat_tex) k_path_tracer<true><<<std::min(path_tracer_grid<true>(), most), kPassBlock, 0, st>>>(s, fp, out);
+        else k_path_tracer<false><<<std::min(path_tracer_grid<false>(), most), kPassBlock, 0, st>>>(s, fp, out);
         MARK(kClsOther);
         return;
     }

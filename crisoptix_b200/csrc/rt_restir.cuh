@@ -307,39 +307,67 @@ RT_D void trace_suffix(const SceneView& s, const FrameParams& fp, Suffix& suffix
     }
 }
 
-// TraceCompletePath (path_gen.h:389-472)
-RT_D V3 trace_complete_path(const SceneView& s, const FrameParams& fp, V3 origin, V3 dir, Rng& rng) {
-    V3 cur_pos = origin, cur_dir = dir;
-    uint32_t depth = 0;
-    V3 radiance = splat(0.0f), tp = splat(1.0f);
-    const float nee = fp.p.nee_prob;
-    for (int ti = 0; ti < fp.p.max_path_len; ++ti) {
+// TraceCompletePath (path_gen.h:389-472) cut at its rays: a lane holds the ray
+// its path waits for, and step() takes the ray's result to the next ray or the
+// end.  The radiance of a light connection does not depend on the shadow ray, so
+// it is evaluated before the ray and the ray only selects between it and zero
+// (a radiance that is bitwise +0 needs no ray).
+struct CompletePath {
+    V3 o, d;        // the ray in flight
+    float tmax;     // 1e16 for an extension ray, the light distance for a shadow ray
+    bool shadow;
+    V3 tp, radiance;
+    uint32_t depth;
+    Rng rng;
+
+    RT_D void begin(V3 origin, V3 dir, const Rng& r) {
+        o = origin;
+        d = dir;
+        tmax = 1e16f;
+        shadow = false;
+        tp = splat(1.0f);
+        radiance = splat(0.0f);
+        depth = 0;
+        rng = r;
+    }
+    // the path's next ray is in o, d, tmax, shadow; false: ended with `radiance`
+    template <bool kTex>
+    RT_D bool step(const SceneView& s, const FrameParams& fp, const TraceResult& h) {
+        if (shadow) {
+            if (h.prim != CRISB_INVALID_PRIM) radiance = splat(0.0f);
+            return false;
+        }
         Isect it;
-        it.valid = false;
-        trace_closest(s, cur_pos, cur_dir, 1e-3f, 1e16f, it);
-        if (!it.valid) break;
+        hit_isect(s, h, d, it);
+        if (!it.valid) return false;
         ++depth;
+        const float nee = fp.p.nee_prob;
         if (rng.next_float() < nee) {
             tp = tp / nee;
             const EmitterSample es = sample_emitter(s, rng);
             const V3 light_dir = normalize(es.pos - it.pos);
             const float dist = length(es.pos - it.pos);
-            if (occluded(s, it.pos, light_dir, 1e-3f, dist)) return splat(0.0f);
-            const BrdfEval be = brdf_eval(s, it, light_dir);
+            const BrdfEval be = brdf_eval<kTex>(s, it, light_dir);
             const float dist_factor = 1.0f / (dist * dist);
             radiance = tp * be.brdf * es.color * dist_factor;
             if (depth == 1) radiance = radiance + be.emission;
-            break;
+            if ((__float_as_uint(radiance.x) | __float_as_uint(radiance.y) | __float_as_uint(radiance.z)) == 0u)
+                return false;
+            o = it.pos;
+            d = light_dir;
+            tmax = dist;
+            shadow = true;
+            return true;
         }
-        const BrdfSample bs = brdf_sample(s, it, rng);
-        if (bs.pdf <= 0.0f) break;
-        cur_pos = it.pos;
-        cur_dir = bs.dir;
+        const BrdfSample bs = brdf_sample<kTex>(s, it, rng);
+        if (bs.pdf <= 0.0f) return false;
         tp = tp * (bs.brdf / bs.pdf);
         tp = tp / (1.0f - nee);
+        o = it.pos;
+        d = bs.dir;
+        return depth < static_cast<uint32_t>(fp.p.max_path_len);
     }
-    return radiance;
-}
+};
 
 // TracePrefixForFinalGather (path_gen.h:474-531)
 RT_D bool trace_prefix_for_gather(const SceneView& s, V3& tp, float& p, Isect& last, V3 origin, V3 dir,

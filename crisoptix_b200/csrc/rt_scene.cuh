@@ -694,6 +694,52 @@ RT_D TraceResult traverse(const SceneView& s, const RayPre& r, float tmin, float
     return traverse_wide4<kAnyHit>(s, r, tmin, tmax);
 }
 
+// The same with the kind of query chosen at run time, for kernels whose lanes
+// trace closest-hit and shadow rays side by side.
+RT_D TraceResult traverse_ray(const SceneView& s, V3 o, V3 d, float tmin, float tmax, bool any) {
+    const RayPre r = make_ray(o, d);
+    if (s.qnodes) {
+        QTrav t;
+        uint4 stk[kQStack];
+        t.init(r, tmin, tmax, any);
+        while (!t.step(s, stk)) {
+        }
+        count_trav(s, t.visits, t.ntris);
+        return t.best;
+    }
+    return any ? traverse_wide4<true>(s, r, tmin, tmax) : traverse_wide4<false>(s, r, tmin, tmax);
+}
+
+// ---- pixels handed to the lanes of persistent warps --------------------------------
+// The warps of a launch take batches of 32 consecutive pixels in turn (warp w the
+// batches w, w + W, ...), and a lane whose path has ended takes the warp's next
+// pixel while the others go on with theirs.  A warp that keeps one path a lane
+// runs until its longest path ends: with 1 to 8 vertices a path, about a third
+// of the lane steps were used.
+struct PixelPool {
+    uint32_t n, warp, warps, next;
+    RT_D PixelPool(uint32_t pixels) {
+        n = pixels;
+        warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        warps = (gridDim.x * blockDim.x) >> 5;
+        next = 0;
+    }
+    // pixel of the warp's v-th place (n or more: none)
+    RT_D uint32_t at(uint32_t v) const {
+        const uint64_t p = (static_cast<uint64_t>(v >> 5) * warps + warp) * 32u + (v & 31u);
+        return p < n ? static_cast<uint32_t>(p) : 0xffffffffu;
+    }
+    // whether pixels are left (uniform over the warp)
+    RT_D bool more() const { return at(next) != 0xffffffffu; }
+    // every lane calls it; a lane with `want` gets its next pixel or 0xffffffff
+    RT_D uint32_t take(bool want) {
+        const unsigned m = __ballot_sync(0xffffffffu, want);
+        const uint32_t v = next + static_cast<uint32_t>(__popc(m & ((1u << (threadIdx.x & 31u)) - 1u)));
+        next += static_cast<uint32_t>(__popc(m));
+        return want ? at(v) : 0xffffffffu;
+    }
+};
+
 // ---- interactions -------------------------------------------------------------
 struct ShadeTri {
     V3 p0, p1, p2, n0, n1, n2;
@@ -719,24 +765,24 @@ RT_HD V3 interp(float bu, float bv, V3 v0, V3 v1, V3 v2) {
     return ((1.0f - bu - bv) * v0) + (bu * v1) + (bv * v2);
 }
 
-// optixTrace + __closesthit__mesh / __miss__main: interaction with the
-// normalised interpolated normal.  On a miss only valid and dir change.
-RT_D void trace_closest(const SceneView& s, V3 o, V3 d, float tmin, float tmax, Isect& it) {
-    count_ray(s, 0);
-    const RayPre r = make_ray(o, d);
-    const TraceResult h = traverse<false>(s, r, tmin, tmax);
+// interaction of a closest hit: position and normalised interpolated normal
+RT_D void hit_isect(const SceneView& s, const TraceResult& h, V3 d, Isect& it) {
     it.dir = d;
-    if (h.prim == CRISB_INVALID_PRIM) {
-        it.valid = false;
-        return;
-    }
-    it.valid = true;
+    it.valid = h.prim != CRISB_INVALID_PRIM;
+    if (!it.valid) return;
     it.prim = h.prim;
     it.bu = h.u;
     it.bv = h.v;
     const ShadeTri t = load_shade(s, h.prim);
     it.pos = interp(it.bu, it.bv, t.p0, t.p1, t.p2);
     it.nrm = normalize(interp(it.bu, it.bv, t.n0, t.n1, t.n2));
+}
+
+// optixTrace + __closesthit__mesh / __miss__main: interaction with the
+// normalised interpolated normal.  On a miss only valid and dir change.
+RT_D void trace_closest(const SceneView& s, V3 o, V3 d, float tmin, float tmax, Isect& it) {
+    count_ray(s, 0);
+    hit_isect(s, traverse<false>(s, make_ray(o, d), tmin, tmax), d, it);
 }
 
 // TraceOcclusion (include/graph/trace.h:64-88)
