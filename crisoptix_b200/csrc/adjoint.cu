@@ -36,26 +36,86 @@ struct AdjView {
     uint32_t num_mats, num_emitters;
 };
 
-// One path of the frozen-sampling estimator; with `sink` also its gradient for
-// the pixel adjoint `dl`.  Returns the pixel's radiance.
+// One path of the frozen-sampling estimator cut at its rays (as CompletePath):
+// a lane holds the ray in flight, step() takes its result to the next ray or the
+// end.  With kGrad the path also adds its gradient for the pixel adjoint `dl`
+// to the sink when it ends in a visible light.
 template <bool kGrad>
-RT_D V3 frozen_path(const AdjView& a, const FrameParams& fp, V3 origin, V3 dir, Rng& rng, V3 dl, GradSink* sink) {
-    SceneView ss = a.eval;  // sampling view: theta0 materials
-    ss.mats = a.sample_mats;
-    V3 cur_pos = origin, cur_dir = dir;
-    uint32_t depth = 0;
-    V3 tp = splat(1.0f);
-    Touched tl[kMaxTouched];
-    int nt = 0;
-    const float nee = fp.p.nee_prob;
-    for (int ti = 0; ti < fp.p.max_path_len; ++ti) {
-        Isect it;
-        it.valid = false;
-        trace_closest(a.eval, cur_pos, cur_dir, 1e-3f, 1e16f, it);
-        if (!it.valid) break;
-        ++depth;
-        const uint32_t mi = material_of(a.eval, it.prim);
+struct FrozenPath {
+    V3 o, d;      // the ray in flight
+    float tmax;   // 1e16 for an extension ray, the light distance for a shadow ray
+    bool shadow;
+    V3 tp, radiance;
+    uint32_t depth;
+    Rng rng;
+    Isect it;     // kGrad: the vertex the shadow ray starts from ...
+    V3 color;     // ... and the light's colour and emitter
+    uint32_t em;
+    int nt;
+
+    RT_D void begin(V3 origin, V3 dir, const Rng& r) {
+        o = origin;
+        d = dir;
+        tmax = 1e16f;
+        shadow = false;
+        tp = splat(1.0f);
+        radiance = splat(0.0f);
+        depth = 0;
+        rng = r;
+        nt = 0;
+    }
+
+    // the light connection's value and, with a sink, its gradient
+    RT_D V3 connect(const AdjView& a, const Isect& v, V3 light_dir, float dist, V3 col, uint32_t ei, V3 dl,
+                    const Touched* tl, GradSink* sink) const {
+        const uint32_t mi = material_of(a.eval, v.prim);
         const crisb_material mat = a.eval.mats[mi];
+        const BrdfGrad bg = brdf_grad(mat, v.nrm, -v.dir, light_dir);
+        const float dist_factor = 1.0f / (dist * dist);
+        V3 r = tp * bg.brdf * col * dist_factor;
+        // brdf_eval reports the emission only past its facing checks
+        const bool emit = depth == 1 && dot(v.nrm, -v.dir) > 0.0f && dot(v.nrm, light_dir) >= 0.0f;
+        if (emit) r = r + mat_vals(mat).emission;
+        if (!kGrad || !sink) return r;
+        const V3 lw = col * dist_factor;  // light weight
+        for (int t = 0; t < nt; ++t) {
+            const V3 c_diff = dl * tl[t].d_diff * bg.brdf * lw;
+            sink->add_mat(tl[t].mat, 0, c_diff.x);
+            sink->add_mat(tl[t].mat, 1, c_diff.y);
+            sink->add_mat(tl[t].mat, 2, c_diff.z);
+            const V3 c_r = dl * tl[t].d_rough * bg.brdf * lw;
+            sink->add_mat(tl[t].mat, 3, (c_r.x + c_r.y) + c_r.z);
+        }
+        const V3 c_diff = dl * tp * bg.d_diff * lw;
+        sink->add_mat(mi, 0, c_diff.x);
+        sink->add_mat(mi, 1, c_diff.y);
+        sink->add_mat(mi, 2, c_diff.z);
+        const V3 c_r = dl * tp * bg.d_rough * lw;
+        sink->add_mat(mi, 3, (c_r.x + c_r.y) + c_r.z);
+        const V3 c_e = dl * tp * bg.brdf * dist_factor;
+        sink->add_em(ei, 0, c_e.x);
+        sink->add_em(ei, 1, c_e.y);
+        sink->add_em(ei, 2, c_e.z);
+        if (emit) {
+            sink->add_mat(mi, 4, dl.x);
+            sink->add_mat(mi, 5, dl.y);
+            sink->add_mat(mi, 6, dl.z);
+        }
+        return r;
+    }
+
+    // the path's next ray is in o, d, tmax, shadow; false: ended with `radiance`
+    RT_D bool step(const AdjView& a, const FrameParams& fp, const TraceResult& h, V3 dl, Touched* tl, GradSink* sink) {
+        if (shadow) {
+            if (h.prim != CRISB_INVALID_PRIM) radiance = splat(0.0f);
+            else if (kGrad) connect(a, it, d, tmax, color, em, dl, tl, sink);
+            return false;
+        }
+        Isect v;
+        hit_isect(a.eval, h, d, v);
+        if (!v.valid) return false;
+        ++depth;
+        const float nee = fp.p.nee_prob;
         if (rng.next_float() < nee) {
             tp = tp / nee;
             if (kGrad)
@@ -64,47 +124,30 @@ RT_D V3 frozen_path(const AdjView& a, const FrameParams& fp, V3 origin, V3 dir, 
                     tl[t].d_rough = tl[t].d_rough / nee;
                 }
             const EmitterSample es = sample_emitter(a.eval, rng);
-            const uint32_t ei = es.index;
-            const V3 light_dir = normalize(es.pos - it.pos);
-            const float dist = length(es.pos - it.pos);
-            if (occluded(a.eval, it.pos, light_dir, 1e-3f, dist)) return splat(0.0f);
-            const BrdfGrad bg = brdf_grad(mat, it.nrm, -it.dir, light_dir);
-            const float dist_factor = 1.0f / (dist * dist);
-            V3 radiance = tp * bg.brdf * es.color * dist_factor;
-            // brdf_eval reports the emission only past its facing checks
-            const bool emit = depth == 1 && dot(it.nrm, -it.dir) > 0.0f && dot(it.nrm, light_dir) >= 0.0f;
-            if (emit) radiance = radiance + mat_vals(mat).emission;
+            const V3 light_dir = normalize(es.pos - v.pos);
+            const float dist = length(es.pos - v.pos);
             if (kGrad) {
-                const V3 lw = es.color * dist_factor;  // light weight
-                for (int t = 0; t < nt; ++t) {
-                    const V3 c_diff = dl * tl[t].d_diff * bg.brdf * lw;
-                    sink->add_mat(tl[t].mat, 0, c_diff.x);
-                    sink->add_mat(tl[t].mat, 1, c_diff.y);
-                    sink->add_mat(tl[t].mat, 2, c_diff.z);
-                    const V3 c_r = dl * tl[t].d_rough * bg.brdf * lw;
-                    sink->add_mat(tl[t].mat, 3, (c_r.x + c_r.y) + c_r.z);
-                }
-                const V3 c_diff = dl * tp * bg.d_diff * lw;
-                sink->add_mat(mi, 0, c_diff.x);
-                sink->add_mat(mi, 1, c_diff.y);
-                sink->add_mat(mi, 2, c_diff.z);
-                const V3 c_r = dl * tp * bg.d_rough * lw;
-                sink->add_mat(mi, 3, (c_r.x + c_r.y) + c_r.z);
-                const V3 c_e = dl * tp * bg.brdf * dist_factor;
-                sink->add_em(ei, 0, c_e.x);
-                sink->add_em(ei, 1, c_e.y);
-                sink->add_em(ei, 2, c_e.z);
-                if (emit) {
-                    sink->add_mat(mi, 4, dl.x);
-                    sink->add_mat(mi, 5, dl.y);
-                    sink->add_mat(mi, 6, dl.z);
-                }
+                it = v;
+                color = es.color;
+                em = es.index;
+            } else {
+                // the value does not depend on the shadow ray: evaluated before it
+                radiance = connect(a, v, light_dir, dist, es.color, es.index, dl, nullptr, nullptr);
+                if ((__float_as_uint(radiance.x) | __float_as_uint(radiance.y) | __float_as_uint(radiance.z)) == 0u)
+                    return false;  // +0 whether or not the light is visible
             }
-            return radiance;
+            o = v.pos;
+            d = light_dir;
+            tmax = dist;
+            shadow = true;
+            return true;
         }
-        const BrdfSample bs = brdf_sample(ss, it, rng);  // direction and pdf at theta0
-        if (bs.pdf <= 0.0f) break;
-        const BrdfGrad bg = brdf_grad(mat, it.nrm, -it.dir, bs.dir);
+        SceneView ss = a.eval;  // sampling view: theta0 materials
+        ss.mats = a.sample_mats;
+        const uint32_t mi = material_of(a.eval, v.prim);
+        const BrdfSample bs = brdf_sample<false>(ss, v, rng);  // direction and pdf at theta0
+        if (bs.pdf <= 0.0f) return false;
+        const BrdfGrad bg = brdf_grad(a.eval.mats[mi], v.nrm, -v.dir, bs.dir);
         const float inv = 1.0f / (bs.pdf * (1.0f - nee));
         const V3 w = bg.brdf * inv;
         if (kGrad) {
@@ -125,44 +168,106 @@ RT_D V3 frozen_path(const AdjView& a, const FrameParams& fp, V3 origin, V3 dir, 
                 tl[slot].d_rough = tl[slot].d_rough + tp * bg.d_rough * inv;
             }
         }
-        cur_pos = it.pos;
-        cur_dir = bs.dir;
+        o = v.pos;
+        d = bs.dir;
         tp = tp * w;
+        return depth < static_cast<uint32_t>(fp.p.max_path_len);
     }
-    return splat(0.0f);
-}
+};
 
-__global__ void __launch_bounds__(kPassBlock) k_frozen_forward(AdjView a, FrameParams fp, float* out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= fp.width * fp.height) return;
-    Rng rng = rng_seeded(tea64(i, fp.random));
-    const V3 dir = camera_dir(fp, i % fp.width, i / fp.width, rng);
-    V3 L = frozen_path<false>(a, fp, ld3(fp.cam.pos), dir, rng, splat(0.0f), nullptr);
-    if (nonfinite(L)) L = splat(0.0f);
-    out[3 * i] = L.x;
-    out[3 * i + 1] = L.y;
-    out[3 * i + 2] = L.z;
-}
-
-__global__ void __launch_bounds__(kPassBlock) k_frozen_backward(AdjView a, FrameParams fp, const float* d_img,
-                                                                float* g_mat, float* g_em, int use_shared) {
-    extern __shared__ float sh[];
-    const uint32_t n_sh = a.num_mats * kMatGrad + a.num_emitters * kEmGrad;
-    if (use_shared) {
-        for (uint32_t k = threadIdx.x; k < n_sh; k += blockDim.x) sh[k] = 0.0f;
-        __syncthreads();
-    }
-    GradSink sink{use_shared ? sh : nullptr, g_mat, g_em, a.num_mats};
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < fp.width * fp.height) {
-        const V3 dl = V3{d_img[3 * i], d_img[3 * i + 1], d_img[3 * i + 2]};
-        if (!nonfinite(dl) && (dl.x != 0.0f || dl.y != 0.0f || dl.z != 0.0f)) {
-            Rng rng = rng_seeded(tea64(i, fp.random));
-            const V3 dir = camera_dir(fp, i % fp.width, i / fp.width, rng);
-            const V3 L = frozen_path<true>(a, fp, ld3(fp.cam.pos), dir, rng, dl, &sink);
-            (void)L;
+// The pixels' paths of a pool: a lane takes the next pixel when its path ends and
+// traces one ray of either kind a turn.  kGrad: `d_img` is the image's adjoint,
+// whose zero and non-finite pixels trace nothing; else `out` is the image.
+template <bool kGrad, class Pool>
+RT_D void frozen_pixels(const AdjView& a, const FrameParams& fp, Pool pool, const float* d_img, float* out,
+                        GradSink* sink) {
+    FrozenPath<kGrad> path;
+    Touched tl[kGrad ? kMaxTouched : 1];
+    V3 dl = splat(0.0f);
+    uint32_t pixel = 0xffffffffu;
+    while (true) {
+        const unsigned idle = __ballot_sync(0xffffffffu, pixel == 0xffffffffu);
+        if (idle) {
+            const bool more = pool.more();
+            if (idle == 0xffffffffu && !more) break;
+            if (more) {
+                const uint32_t i = pool.take(pixel == 0xffffffffu);
+                bool start = i != 0xffffffffu;
+                if (kGrad && start) {
+                    dl = V3{d_img[3 * i], d_img[3 * i + 1], d_img[3 * i + 2]};
+                    start = !nonfinite(dl) && (dl.x != 0.0f || dl.y != 0.0f || dl.z != 0.0f);
+                }
+                if (start) {
+                    pixel = i;
+                    Rng rng = rng_seeded(tea64(i, fp.random));
+                    const V3 dir = camera_dir(fp, i % fp.width, i / fp.width, rng);
+                    path.begin(ld3(fp.cam.pos), dir, rng);
+                }
+            }
+        }
+        if (pixel != 0xffffffffu) {
+            const TraceResult h = traverse_ray(a.eval, path.o, path.d, 1e-3f, path.tmax, path.shadow);
+            if (!path.step(a, fp, h, dl, tl, sink)) {
+                if (!kGrad) {
+                    V3 L = path.radiance;
+                    if (nonfinite(L)) L = splat(0.0f);
+                    out[3 * pixel] = L.x;
+                    out[3 * pixel + 1] = L.y;
+                    out[3 * pixel + 2] = L.z;
+                }
+                pixel = 0xffffffffu;
+            }
         }
     }
+}
+
+// 6 resident blocks per SM (80 registers; 4 and 5 blocks: 2-4% slower)
+__global__ void __launch_bounds__(kPassBlock, 6) k_frozen_forward(AdjView a, FrameParams fp, float* out) {
+    frozen_pixels<false>(a, fp, PixelPool(fp.width * fp.height), nullptr, out, nullptr);
+}
+
+// Backward: a block of two warps per group of 128 pixels, whose lanes take the
+// group's pixels in turn and whose gradients gather in one shared-memory block of
+// all parameters (12 KB for the large scene) that reaches global memory once.
+// The group, not the block, sets how the gradients' float sums are split:
+// larger ones, as persistent warps would have, change them by 2e-5 through what a
+// global sum of 1e9 takes from each addition.  Forward and backward of 8 views of
+// 512 x 512: 11.3 ms with 64 threads a group (10 blocks per SM, 96 registers), 12.3
+// with 128, 11.9 with 96, 11.7 with 32; 15.9 with a thread a pixel, each warp
+// running until its longest path ended.
+constexpr uint32_t kGroup = 128;
+constexpr int kGroupThreads = 64;
+
+// the pixels of a block's group, taken by its lanes in turn
+struct GroupPool {
+    uint32_t first, count;
+    uint32_t* taken;  // shared
+    RT_D bool more() const {
+        const uint32_t t = __shfl_sync(0xffffffffu, *static_cast<volatile uint32_t*>(taken), 0);
+        return t < count;
+    }
+    RT_D uint32_t take(bool want) {
+        const unsigned m = __ballot_sync(0xffffffffu, want);
+        const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+        uint32_t v = 0;
+        if (lane == leader) v = atomicAdd(taken, static_cast<uint32_t>(__popc(m)));
+        v = __shfl_sync(0xffffffffu, v, leader) + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
+        return want && v < count ? first + v : 0xffffffffu;
+    }
+};
+
+__global__ void __launch_bounds__(kGroupThreads, 10) k_frozen_backward(AdjView a, FrameParams fp, const float* d_img,
+                                                                      float* g_mat, float* g_em, int use_shared) {
+    extern __shared__ float sh[];
+    __shared__ uint32_t taken;
+    const uint32_t n_sh = a.num_mats * kMatGrad + a.num_emitters * kEmGrad;
+    if (threadIdx.x == 0) taken = 0;
+    if (use_shared)
+        for (uint32_t k = threadIdx.x; k < n_sh; k += blockDim.x) sh[k] = 0.0f;
+    __syncthreads();
+    GradSink sink{use_shared ? sh : nullptr, g_mat, g_em, a.num_mats};
+    const uint32_t first = blockIdx.x * kGroup;
+    frozen_pixels<true>(a, fp, GroupPool{first, min(kGroup, fp.width * fp.height - first), &taken}, d_img, nullptr, &sink);
     if (use_shared) {
         __syncthreads();
         for (uint32_t k = threadIdx.x; k < n_sh; k += blockDim.x) {
@@ -174,6 +279,17 @@ __global__ void __launch_bounds__(kPassBlock) k_frozen_backward(AdjView a, Frame
     }
 }
 
+// blocks of `kernel` resident on the device at once
+unsigned resident_blocks(const void* kernel) {
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPassBlock, 0) == cudaSuccess && sms > 0 &&
+        per_sm > 0)
+        return static_cast<unsigned>(sms * per_sm);
+    return 148u * 4u;
+}
+
 }  // namespace
 
 // host side, called from api.cu
@@ -181,7 +297,8 @@ void adjoint_forward(const SceneView& eval, const crisb_material* sample_mats, u
                      const FrameParams& fp, float* out, cudaStream_t st) {
     const AdjView a{eval, sample_mats, num_mats, eval.num_emitters};
     const uint32_t P = fp.width * fp.height;
-    k_frozen_forward<<<(P + kPassBlock - 1) / kPassBlock, kPassBlock, 0, st>>>(a, fp, out);
+    static const unsigned resident = resident_blocks(reinterpret_cast<const void*>(k_frozen_forward));
+    k_frozen_forward<<<std::min((P + kPassBlock - 1) / kPassBlock, resident), kPassBlock, 0, st>>>(a, fp, out);
 }
 
 void adjoint_backward(const SceneView& eval, const crisb_material* sample_mats, uint32_t num_mats,
@@ -190,8 +307,8 @@ void adjoint_backward(const SceneView& eval, const crisb_material* sample_mats, 
     const uint32_t P = fp.width * fp.height;
     const size_t sh_bytes = (static_cast<size_t>(num_mats) * kMatGrad + eval.num_emitters * kEmGrad) * sizeof(float);
     const int use_shared = sh_bytes <= 48u * 1024u ? 1 : 0;
-    k_frozen_backward<<<(P + kPassBlock - 1) / kPassBlock, kPassBlock, use_shared ? sh_bytes : 0, st>>>(
-        a, fp, d_img, g_mat, g_em, use_shared);
+    const size_t shb = use_shared ? sh_bytes : 0;
+    k_frozen_backward<<<(P + kGroup - 1) / kGroup, kGroupThreads, shb, st>>>(a, fp, d_img, g_mat, g_em, use_shared);
 }
 
 }  // namespace crisb
