@@ -714,7 +714,7 @@ struct crisb_renderer {
         b.pass_flags = pass_flags.p;
         b.spatial_nbr = spatial_nbr.p;
         b.job_items = job_items.p;
-        b.job_count = nullptr;  // job_count, wf_count and job_qcount: taken by each pass
+        b.job_count = nullptr;  // job_count, path_counts, path_next and job_qcount: taken by each pass
         b.shift_out = shift_out.p;
         b.gather_cs = gather_cs.p;
         b.gather_state = gather_state.p;
@@ -723,9 +723,9 @@ struct crisb_renderer {
         b.slots = slots;
         b.job_cap = static_cast<uint32_t>(std::min<size_t>(job_capacity(), 0xFFFFFFFFu));
         b.tally = timing >= 2 && ray_count.p ? ray_count.p + kRayCounters : nullptr;
-        b.wf = reinterpret_cast<WfPath*>(machine_state.p);
-        for (int q = 0; q < 4; ++q) b.wf_queue[q] = machine_queue[q].p;
-        b.wf_count = nullptr;
+        b.paths = reinterpret_cast<PathState*>(machine_state.p);
+        for (int q = 0; q < 4; ++q) b.path_queue[q] = machine_queue[q].p;
+        b.path_counts = b.path_next = nullptr;
         b.gather_cp = gather_cp.p;
         b.jobs = reinterpret_cast<ShiftJob*>(machine_state.p);
         for (int q = 0; q < 4; ++q) b.job_queue[q] = machine_queue[q].p;
@@ -780,7 +780,7 @@ struct crisb_renderer {
         spatial_nbr.alloc(p * (slots / 2));
         job_items.alloc(p * slots);
         shift_out.alloc(p * slots);
-        const size_t state = std::max(p * sizeof(WfPath), job_capacity() * sizeof(ShiftJob));
+        const size_t state = std::max(p * sizeof(PathState), job_capacity() * sizeof(ShiftJob));
         machine_state.alloc((state + 255) & ~static_cast<size_t>(255));
         for (int q = 0; q < 4; ++q) machine_queue[q].alloc(std::max(p, job_capacity()));
     }
@@ -926,10 +926,7 @@ struct crisb_renderer {
         fp.back = back;
         fp.k = K();
         fp.trace_grid = std::max(1u, trace_grid / std::max(1u, concurrent_views));
-        // views rendering at once keep shared memory out of their init kernels:
-        // the 16-view batch ran 100.7 ms per frame with the staged instances
-        // beside 95.7 without, while a single 1080p view gains 0.17 ms from them
-        fp.shared_stage = concurrent_views > 1 ? 0u : 1u;
+        fp.concurrent = concurrent_views > 1 ? 1u : 0u;
         fp.trace_block = trace_block;
         require(params.motion_mode != CRISB_MOTION_VECTORS || motion != nullptr,
                 "render_frame: CRISB_MOTION_VECTORS without motion vectors");
@@ -963,7 +960,7 @@ struct crisb_renderer {
         launch_prefix_gen_temp_split(s, fp, bufs(), cn, out, st, m);
         launches += params.renderer_type == CRISB_RENDERER_PATH_TRACER
                         ? 1
-                        : 2 + shift_launches(params, kModePrefix) + wf_launches_per_pass(fp, 0) +
+                        : 2 + flow_launches(fp, 0, scene->textured) + shift_launches(params, kModePrefix) +
                               prefix_pass_extra_launches(fp);
         record(1, st);
         const int type = params.renderer_type;
@@ -985,7 +982,7 @@ struct crisb_renderer {
         if (type == CRISB_RENDERER_CONDITIONAL_RESTIR) {
             launch_suffix_gen_temp(s, fp, bufs(), cn, st, m);
             scur ^= 1;
-            launches += 2 + shift_launches(params, kModeTemporal) + wf_launches_per_pass(fp, 1);
+            launches += 2 + flow_launches(fp, 1, scene->textured) + shift_launches(params, kModeTemporal);
             record(3, st);
             if (params.suffix_enable_spatial && params.suffix_spatial_count > 0) {
                 for (int r = 0; r < params.suffix_spatial_rounds; ++r) {
@@ -1011,7 +1008,7 @@ struct crisb_renderer {
                 gather_last.alloc(P());
             }
             launch_final_gather_split(s, fp, bufs(), cn, out, st, m);
-            launches += 1 + wf_launches_per_pass(fp, 2);
+            launches += 1 + flow_launches(fp, 2, scene->textured);
             if (K() > 0) launches += 2 + shift_launches(params, kModeGather);
             if (params.gather_n > 1)
                 launches += 1 + static_cast<uint32_t>(params.gather_n - 1) * (3 + shift_launches(params, kModeGatherExtra));

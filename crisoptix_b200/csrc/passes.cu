@@ -146,7 +146,7 @@ void launch_prefix_copy_front_back(const FrameParams& fp, const Bufs& b, cudaStr
 void launch_store_entries(const SceneView& s, const FrameParams& fp, const Bufs& b, const lbvh::Work& w,
                           unsigned int* bounds, cudaStream_t st) {
     k_bounds_init<<<1, 32, 0, st>>>(bounds, w.n);
-    if (fp.shared_stage) k_store_entries<true><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b, s, bounds, w.n);
+    if (!fp.concurrent) k_store_entries<true><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b, s, bounds, w.n);
     else k_store_entries<false><<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b, s, bounds, w.n);
     k_knn_keys<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b, w, bounds);
 }

@@ -5,7 +5,6 @@
 
 #include "knn.cuh"
 #include "rt_restir.cuh"
-#include "wavefront.cuh"
 
 namespace crisb {
 
@@ -21,6 +20,13 @@ struct ShiftJob {
     uint64_t rng;  // replay RNG of the source path
     uint32_t code; // job code: pixel << 6 | slot
     uint32_t ctr;  // replays left after the ray in flight
+};
+
+// State of a path between two launches of its flow (160 bytes; a path waiting
+// for an extension ray uses the first 80 and the ray's result)
+struct PathState {
+    uint4 w[9];  // FlowPath::save
+    uint4 hit;   // the ray's result: triangle, t, u, v (a shadow ray's: triangle alone)
 };
 
 // A reservoir buffer in one of the two storage layouts: crisb_*_res_rec
@@ -87,11 +93,13 @@ struct Bufs {
     // statistics level 2 only (else null): bytes read and written by each
     // resampling kernel for the work present in the frame (kTally*)
     unsigned long long* tally;
-    // wavefront path tracing: one path state per pixel, ray queues of two
-    // rounds (closest, shadow) x 2 and the counts of every round of the pass
-    WfPath* wf;
-    uint32_t* wf_queue[4];
-    uint32_t* wf_count;          // 2 per round (Counters)
+    // path flows: the states of paths between launches, ray queues of two rounds
+    // (closest, shadow) x 2, and the counts of every round of the pass and the
+    // next item of its persistent launch
+    PathState* paths;            // P
+    uint32_t* path_queue[4];     // P each
+    uint32_t* path_counts;       // 2 per round (Counters)
+    uint32_t* path_next;         // 1 (Counters)
     crisb_prefix_rec* gather_cp; // canonical prefix of the final gather
     // shift machines: one record per job of the list, ray queues of two
     // rounds (closest, shadow) x 2 and the counts of every round of the phase
@@ -114,7 +122,7 @@ enum KernelClass : int {
     kClsShade = 5,     // path-machine shading steps and per-pass finish kernels
 };
 
-// pass_status of a pixel after a wavefront init kernel
+// pass_status of a pixel after a path flow
 constexpr uint32_t kWfIdle = 0;  // no path ran for the pixel
 constexpr uint32_t kWfPath = 4;  // a path ran for the pixel
 
@@ -161,14 +169,14 @@ void launch_suffix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Co
                            Marker* m);
 void launch_final_gather_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                cudaStream_t st, Marker* m);
-// wavefront path tracing (wavefront.cu): init + rounds of trace / shade;
-// b.wf_count holds 2 x wf_round_count cleared counters
-int wf_round_count(const crisb_params& p, int flow);
+// the path flows of a pass (wavefront.cu)
+constexpr int kMaxFlowRounds = 8;
+int flow_rounds(const FrameParams& fp, int flow, bool textured);
+// kernels of one path flow (0 prefix, 1 suffix, 2 gather)
+uint32_t flow_launches(const FrameParams& fp, int flow, bool textured);
 void launch_wf_prefix(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
 void launch_wf_suffix(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
 void launch_wf_gather(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
-// kernels of one wavefront pass of `flow` (0 prefix, 1 suffix, 2 gather)
-uint32_t wf_launches_per_pass(const FrameParams& fp, int flow);
 // kernels of one shift-job phase (begin + rounds of closest / shadow / step)
 uint32_t shift_launches(const crisb_params& p, int mode);
 // what a shift phase shifts (the job's source and destination)

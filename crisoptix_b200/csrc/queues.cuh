@@ -27,21 +27,20 @@ RT_D void q_append(uint32_t* q, uint32_t* cnt, bool take, uint32_t val) {
     if (take) q[base + __popc(mask & ((1u << lane) - 1u))] = val;
 }
 
-// path machine records: next closest-hit ray in ray_o / ray_d, the NEE shadow
-// ray from it_pos along nee_dir (w = light distance)
-RT_D void closest_ray(const WfPath& w, V3& o, V3& d) {
-    const float4 a = w.ray_o, b = w.ray_d;
-    o = V3{a.x, a.y, a.z};
-    d = V3{b.x, b.y, b.z};
+// path states (FlowPath::save): a shadow ray's result is a triangle if occluded
+RT_D void closest_ray(const PathState& p, V3& o, V3& d) {
+    const uint4 a = p.w[1], b = p.w[2];
+    o = V3{__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z)};
+    d = V3{__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z)};
 }
-RT_D void set_hit(WfPath& w, float4 h) { w.hit = h; }
-RT_D void shadow_ray(const WfPath& w, V3& o, V3& d, float& tmax) {
-    const float4 a = w.it_pos, b = w.nee_dir;
-    o = V3{a.x, a.y, a.z};
-    d = V3{b.x, b.y, b.z};
-    tmax = b.w;
+RT_D void set_hit(PathState& p, float4 h) {
+    p.hit = make_uint4(__float_as_uint(h.x), __float_as_uint(h.y), __float_as_uint(h.z), __float_as_uint(h.w));
 }
-RT_D void set_occluded(WfPath& w, uint32_t v) { w.occluded = v; }
+RT_D void shadow_ray(const PathState& p, V3& o, V3& d, float& tmax) {
+    closest_ray(p, o, d);
+    tmax = __uint_as_float(p.w[5].x);
+}
+RT_D void set_occluded(PathState& p, uint32_t v) { p.hit.x = v ? 0u : CRISB_INVALID_PRIM; }
 
 // shift machine records: one ray in flight in o / d
 RT_D void closest_ray(const ShiftJob& j, V3& o, V3& d) {

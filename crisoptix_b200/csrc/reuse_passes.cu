@@ -24,6 +24,11 @@
 namespace crisb {
 namespace {
 
+enum RayRequest : int { kReqDone = 0, kReqClosest = 1, kReqShadow = 2 };
+
+RT_D V3 f3(float4 v) { return V3{v.x, v.y, v.z}; }
+RT_D float4 f4(V3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
+
 constexpr uint32_t kStFinal = 0;      // nothing left to do in the combine kernel
 constexpr uint32_t kStCanonOnly = 1;  // temporal: stream the canonical sample only
 constexpr uint32_t kStReuse = 2;      // reuse with the shift results
@@ -379,8 +384,7 @@ __global__ void __launch_bounds__(kPassBlock) k_suffix_temp_finish(FrameParams f
     uint64_t mask = 0;
     if (i < pixel_count(fp)) {
         uint32_t st = kStFinal;
-        if (b.pass_status[i] == kWfPath) {  // else the init kernel invalidated the reservoir
-            b.gbuf[i].rng = b.wf[i].rng;
+        if (b.pass_status[i] == kWfPath) {  // else the flow invalidated the reservoir
             const uint32_t prev_xy = b.gbuf[i].prev_xy;
             if (!fl_valid(b.canon_suffix[i].sample.flags)) {
                 Res<Suffix> cur = ld_sres(b.sres_cur, i);
@@ -616,7 +620,6 @@ __global__ void __launch_bounds__(kPassBlock) k_gather_finish(FrameParams fp, Bu
     V3 direct = splat(0.0f);
     if (fp.k == 0) b.neigh_count[i] = 0;  // no query runs
     if (b.pass_status[i] == kWfPath) {
-        b.gbuf[i].rng = b.wf[i].rng;
         const Prefix cp = ld_prefix_v(b.gather_cp[i]);
         if (fl_valid(cp.flags)) {
             if (fl_nee(cp.flags)) {
@@ -1045,7 +1048,7 @@ __global__ void __launch_bounds__(kPassBlock) k_prefix_finish(SceneView s, Frame
             }
         }
         crisb_gbuffer_rec g;
-        g.rng = b.wf[i].rng;
+        g.rng = b.gbuf[i].rng;
         g.prev_xy = prev_xy;
         g.flags = valid ? 1u : 0u;
         b.gbuf[i] = g;
@@ -1162,12 +1165,12 @@ int shift_rounds(const crisb_params& p, int mode) {
     return std::min(std::max(len - 1, 1), kShiftRounds);
 }
 
-// the counters of one shift phase and, with `rounds` > 0, a wavefront pass
-void take_counters(Bufs& b, Counters& c, int rounds) {
-    // max_path_len <= 255 keeps a pass well below the array's size
-    uint32_t* p = c.take(2 * static_cast<uint32_t>(rounds) + 1 + 2 * kShiftRounds);
-    b.wf_count = p;
-    b.job_count = p + 2 * rounds;
+// the counters of one path flow and one shift phase
+void take_counters(Bufs& b, Counters& c) {
+    uint32_t* p = c.take(2 * (kMaxFlowRounds + 1) + 2 + 2 * kShiftRounds);
+    b.path_counts = p;
+    b.path_next = p + 2 * (kMaxFlowRounds + 1);
+    b.job_count = b.path_next + 1;
     b.job_qcount = b.job_count + 1;
 }
 
@@ -1221,7 +1224,7 @@ void launch_prefix_gen_temp_split(const SceneView& s, const FrameParams& fp, Buf
         MARK(kClsOther);
         return;
     }
-    take_counters(b, c, wf_round_count(fp.p, 0));
+    take_counters(b, c);
     launch_wf_prefix(s, fp, b, st, m);
     k_prefix_finish<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b, out);
     MARK(kClsShade);
@@ -1240,7 +1243,7 @@ uint32_t prefix_pass_extra_launches(const FrameParams& fp) {
 
 void launch_prefix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out, int round,
                            cudaStream_t st, Marker* m) {
-    take_counters(b, c, 0);
+    take_counters(b, c);
     k_prefix_spatial_select<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     MARK(kClsResample);
     run_shift_jobs(s, fp, b, kModePrefixSpatial, st, m);
@@ -1250,7 +1253,7 @@ void launch_prefix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Co
 
 void launch_suffix_gen_temp(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, cudaStream_t st,
                             Marker* m) {
-    take_counters(b, c, wf_round_count(fp.p, 1));
+    take_counters(b, c);
     launch_wf_suffix(s, fp, b, st, m);
     k_suffix_temp_finish<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     MARK(kClsShade);
@@ -1261,7 +1264,7 @@ void launch_suffix_gen_temp(const SceneView& s, const FrameParams& fp, Bufs b, C
 
 void launch_suffix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, cudaStream_t st,
                            Marker* m) {
-    take_counters(b, c, 0);
+    take_counters(b, c);
     k_suffix_spatial_select<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b);
     MARK(kClsResample);
     run_shift_jobs(s, fp, b, kModeSpatial, st, m);
@@ -1271,7 +1274,7 @@ void launch_suffix_spatial(const SceneView& s, const FrameParams& fp, Bufs b, Co
 
 void launch_final_gather_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                cudaStream_t st, Marker* m) {
-    take_counters(b, c, wf_round_count(fp.p, 2));
+    take_counters(b, c);
     launch_wf_gather(s, fp, b, st, m);
     k_gather_finish<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(fp, b, out);
     MARK(kClsShade);
@@ -1284,7 +1287,7 @@ void launch_final_gather_split(const SceneView& s, const FrameParams& fp, Bufs b
     }
     if (fp.p.gather_n > 1) {
         for (int g = 1; g < fp.p.gather_n; ++g) {
-            take_counters(b, c, 0);
+            take_counters(b, c);
             k_gather_extra_prefix<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b);
             MARK(kClsShade);
             k_gather_extra_query<<<grid_for(fp.width * fp.height), kPassBlock, 0, st>>>(s, fp, b);

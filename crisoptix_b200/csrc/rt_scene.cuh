@@ -740,6 +740,44 @@ struct PixelPool {
     }
 };
 
+// Work items [0, n) handed out through a counter in global memory (cleared before
+// the launch), 32 consecutive ones to a warp at a time, and from there to its
+// lanes as they fall idle: blocks that start late, beside other launches, find
+// less to do instead of a share of their own.
+struct WorkPool {
+    uint32_t n;
+    uint32_t* counter;
+    uint32_t base, left;  // the warp's current batch
+    bool open;            // the counter may have more
+    RT_D WorkPool(uint32_t items, uint32_t* next) : n(items), counter(next), base(0), left(0), open(items > 0) {}
+    // uniform over the warp
+    RT_D bool more() const { return left > 0 || open; }
+    // every lane calls it; a lane with `want` gets an item or 0xffffffff
+    RT_D uint32_t take(bool want) {
+        const unsigned m = __ballot_sync(0xffffffffu, want);
+        const uint32_t lane = threadIdx.x & 31u;
+        const uint32_t k = static_cast<uint32_t>(__popc(m));
+        const uint32_t rank = static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
+        uint32_t item = rank < left ? base + rank : 0xffffffffu;
+        if (k <= left) {
+            base += k;
+            left -= k;
+        } else {
+            const uint32_t over = rank - left;
+            uint32_t nb = 0;
+            if (lane == 0 && open) nb = atomicAdd(counter, 32u);
+            nb = __shfl_sync(0xffffffffu, nb, 0);
+            const uint32_t c = open && nb < n ? min(32u, n - nb) : 0u;
+            if (c == 0) open = false;
+            if (rank >= left && over < c) item = nb + over;
+            const uint32_t used = min(k - left, c);
+            base = nb + used;
+            left = c - used;
+        }
+        return want ? item : 0xffffffffu;
+    }
+};
+
 // ---- interactions -------------------------------------------------------------
 struct ShadeTri {
     V3 p0, p1, p2, n0, n1, n2;
