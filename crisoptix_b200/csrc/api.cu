@@ -714,7 +714,7 @@ struct crisb_renderer {
         b.pass_flags = pass_flags.p;
         b.spatial_nbr = spatial_nbr.p;
         b.job_items = job_items.p;
-        b.job_count = nullptr;  // job_count, path_counts, path_next and job_qcount: taken by each pass
+        b.job_count = nullptr;  // job_count, path_counts, path_next, job_qcount, job_next: taken by each pass
         b.shift_out = shift_out.p;
         b.gather_cs = gather_cs.p;
         b.gather_state = gather_state.p;
@@ -729,7 +729,7 @@ struct crisb_renderer {
         b.gather_cp = gather_cp.p;
         b.jobs = reinterpret_cast<ShiftJob*>(machine_state.p);
         for (int q = 0; q < 4; ++q) b.job_queue[q] = machine_queue[q].p;
-        b.job_qcount = nullptr;
+        b.job_qcount = b.job_next = nullptr;
         return b;
     }
 
@@ -960,7 +960,7 @@ struct crisb_renderer {
         launch_prefix_gen_temp_split(s, fp, bufs(), cn, out, st, m);
         launches += params.renderer_type == CRISB_RENDERER_PATH_TRACER
                         ? 1
-                        : 2 + flow_launches(fp, 0, scene->textured) + shift_launches(params, kModePrefix) +
+                        : 2 + flow_launches(fp, 0, scene->textured) + shift_launches(fp) +
                               prefix_pass_extra_launches(fp);
         record(1, st);
         const int type = params.renderer_type;
@@ -975,19 +975,19 @@ struct crisb_renderer {
                 launch_prefix_spatial(s, fp, bufs(), cn, out, r, st, m);
                 launch_prefix_copy_front_back(fp, bufs(), st);
                 if (m) m->mark(kClsOther, st);
-                launches += 3 + shift_launches(params, kModePrefixSpatial);
+                launches += 3 + shift_launches(fp);
             }
         }
         record(2, st);
         if (type == CRISB_RENDERER_CONDITIONAL_RESTIR) {
             launch_suffix_gen_temp(s, fp, bufs(), cn, st, m);
             scur ^= 1;
-            launches += 2 + flow_launches(fp, 1, scene->textured) + shift_launches(params, kModeTemporal);
+            launches += 2 + flow_launches(fp, 1, scene->textured) + shift_launches(fp);
             record(3, st);
             if (params.suffix_enable_spatial && params.suffix_spatial_count > 0) {
                 for (int r = 0; r < params.suffix_spatial_rounds; ++r) {
                     launch_suffix_spatial(s, fp, bufs(), cn, st, m);
-                    launches += 2 + shift_launches(params, kModeSpatial);
+                    launches += 2 + shift_launches(fp);
                     scur ^= 1;
                 }
             }
@@ -1009,9 +1009,9 @@ struct crisb_renderer {
             }
             launch_final_gather_split(s, fp, bufs(), cn, out, st, m);
             launches += 1 + flow_launches(fp, 2, scene->textured);
-            if (K() > 0) launches += 2 + shift_launches(params, kModeGather);
+            if (K() > 0) launches += 2 + shift_launches(fp);
             if (params.gather_n > 1)
-                launches += 1 + static_cast<uint32_t>(params.gather_n - 1) * (3 + shift_launches(params, kModeGatherExtra));
+                launches += 1 + static_cast<uint32_t>(params.gather_n - 1) * (3 + shift_launches(fp));
         } else {
             record(3, st);
             record(4, st);

@@ -88,7 +88,7 @@ struct Bufs {
     float4* gather_state;   // P * 3: prefix f / p, canonical contribution, direct result
     uint32_t slots;         // job slots per pixel (>= 2 * max(k, spatial count, 1))
     // capacity of the shift machines' job records and queues; list entries
-    // beyond it run in k_shift_overflow, tracing their rays in place
+    // beyond it start on the phase's persistent warps
     uint32_t job_cap;
     // statistics level 2 only (else null): bytes read and written by each
     // resampling kernel for the work present in the frame (kTally*)
@@ -106,6 +106,7 @@ struct Bufs {
     ShiftJob* jobs;         // P * slots
     uint32_t* job_queue[4]; // P * slots each
     uint32_t* job_qcount;   // 2 per round (Counters)
+    uint32_t* job_next;     // 1: next item of the persistent launch (Counters)
 
     RT_HD KnnView knn() const { return KnnView{knn_nodes, knn_leaf, knn_pixel, knn_n}; }
 };
@@ -177,8 +178,9 @@ uint32_t flow_launches(const FrameParams& fp, int flow, bool textured);
 void launch_wf_prefix(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
 void launch_wf_suffix(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
 void launch_wf_gather(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m);
-// kernels of one shift-job phase (begin + rounds of closest / shadow / step)
-uint32_t shift_launches(const crisb_params& p, int mode);
+// kernels of one shift-job phase
+constexpr int kMaxShiftRounds = 4;
+uint32_t shift_launches(const FrameParams& fp);
 // what a shift phase shifts (the job's source and destination)
 enum ShiftMode : int {
     kModeTemporal = 0,  // suffix temporal reuse

@@ -24,9 +24,9 @@
 namespace crisb {
 namespace {
 
-enum RayRequest : int { kReqDone = 0, kReqClosest = 1, kReqShadow = 2 };
+// what a shift job waits for
+enum JobPhase : uint32_t { kJobDone = 0, kJobStart = 1, kJobHit = 2, kJobShadow = 3 };
 
-RT_D V3 f3(float4 v) { return V3{v.x, v.y, v.z}; }
 RT_D float4 f4(V3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
 
 constexpr uint32_t kStFinal = 0;      // nothing left to do in the combine kernel
@@ -83,11 +83,7 @@ RT_D void count_jobs(const SceneView& s, uint32_t total) {
 // shifted contribution do not depend on the visibility result, so they are
 // evaluated before the shadow ray is queued and the ray only selects between
 // them and zero -- the value the per-job function returns when the edge is
-// occluded.  Jobs that still need a replay in the last round finish inline.
-// Three rounds: 4 / 5 / 6 rounds cut the shift steps from 1.46 to 1.40 / 1.27
-// / 1.20 ms per 1080p frame but added more in traversal launches (frame 17.04
-// -> 17.20 / 17.32 / 17.35 ms).
-constexpr int kShiftRounds = 3;
+// occluded.
 RT_HD bool prefix_mode(int mode) { return mode == kModePrefix || mode == kModePrefixSpatial; }
 
 // source path of a job
@@ -167,212 +163,251 @@ RT_D void job_out(const Bufs& b, uint32_t code, float4 v) {
     b.shift_out[static_cast<size_t>(i) * b.slots + slot] = v;
 }
 
-// Runs the job from vertex `cur` with `left` replays to go: queues its next
-// ray (returned request) or, when `inline_rays`, traces the remaining rays in
-// place; a finished job writes its result.
-template <bool kTex>
-RT_D int shift_advance(const SceneView& s, const Bufs& b, bool prefix, const ShiftSrc& src, ShiftJob& j, Isect cur,
-                       Rng& srng, V3 tp, uint32_t left, bool inline_rays) {
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    while (left > 0) {
-        srng.next_float();
-        const BrdfSample bs = brdf_sample<kTex>(s, cur, srng);
-        if (bs.pdf <= 0.0f) {
-            job_out(b, j.code, zero);
-            return kReqDone;
-        }
-        tp = tp * bs.brdf;
-        --left;
-        if (!inline_rays) {
-            j.o = f4(cur.pos, 0.0f);
-            j.d = f4(bs.dir, 0.0f);
-            j.acc = f4(tp, 0.0f);
-            j.rng = srng.state;
-            j.ctr = left;
-            return kReqClosest;
-        }
-        const V3 pos = cur.pos;
-        trace_closest(s, pos, bs.dir, 1e-3f, 1e16f, cur);
-        if (!cur.valid) {
-            job_out(b, j.code, zero);
-            return kReqDone;
-        }
-    }
-    // the reconnection edge
-    const Isect src_anchor = unpack(s, src.anchor);
-    Isect src_recon = unpack(s, src.recon);
-    const V3 rv = src_recon.pos - cur.pos;
-    const float rlen = length(rv);
-    const V3 rdir = normalize(rv);
-    if ((prefix && isinf(rlen)) || nonfinite(rdir)) {
-        job_out(b, j.code, zero);
-        return kReqDone;
-    }
-    const BrdfEval b1 = brdf_eval<kTex>(s, cur, rdir);
-    float4 res = zero;
-    if (b1.pdf > 0.0f) {
-        tp = tp * b1.brdf;
-        bool ok = true;
-        if (prefix || fl_recon(src.flags) < fl_len(src.flags)) {
-            src_recon.dir = rdir;
-            if (!prefix && is_zero(src.rod)) ok = false;
-            if (ok) {
-                const BrdfEval b2 = brdf_eval<kTex>(s, src_recon, src.rod);
-                if (b2.pdf <= 0.0f) ok = false;
-                else tp = tp * b2.brdf;
-            }
-        }
-        if (ok) {
-            const float jac = recon_jacobian(src_anchor.pos, cur.pos, src_recon.pos, src_recon.nrm);
-            const V3 f = prefix ? gmax(splat(0.0f), tp * src.prf) : tp * src.prf;
-            res = f4(f, jac);
-        }
-    }
-    if ((__float_as_uint(res.x) | __float_as_uint(res.y) | __float_as_uint(res.z) | __float_as_uint(res.w)) == 0u) {
-        job_out(b, j.code, zero);  // +0 whether or not the edge is visible
-        return kReqDone;
-    }
-    if (inline_rays) {
-        job_out(b, j.code, occluded(s, cur.pos, rdir, 1e-3f, rlen) ? zero : res);
-        return kReqDone;
-    }
-    j.o = f4(cur.pos, rlen);
-    j.d = f4(rdir, 0.0f);
-    j.acc = res;
-    return kReqShadow;
-}
-
-// a job waiting for its ray: everything but the hit word, which the traversal
-// kernels write
-RT_D void job_store(ShiftJob* r, const ShiftJob& j) {
-    r->o = j.o;
-    r->d = j.d;
-    r->acc = j.acc;
-    r->rng = j.rng;
-    r->code = j.code;
-    r->ctr = j.ctr;
-}
-
 // queue job t's ray for round `round` (two queue pairs, used in turn)
-RT_D void job_push(const Bufs& b, int round, int req, uint32_t t) {
+RT_D void job_push(const Bufs& b, int round, uint32_t phase, uint32_t t) {
     const int q = 2 * (round & 1);
-    q_append(b.job_queue[q], &b.job_qcount[2 * round], req == kReqClosest, t);
-    q_append(b.job_queue[q + 1], &b.job_qcount[2 * round + 1], req == kReqShadow, t);
+    q_append(b.job_queue[q], &b.job_qcount[2 * round], phase == kJobHit, t);
+    q_append(b.job_queue[q + 1], &b.job_qcount[2 * round + 1], phase == kJobShadow, t);
 }
 
-// first step of every job of the list: the checks of the reference function,
-// then the first ray
+// A lane's job.  step() starts it (its source and destination vertex and the
+// checks of the reference function) or takes its ray's result to the next ray
+// or the end, which writes the result.
 // kTex: the scene has textured materials
 template <bool kTex>
-__global__ void __launch_bounds__(kPassBlock) k_shift_begin(SceneView s, FrameParams fp, Bufs b, int mode) {
-    const uint32_t all = *b.job_count;
-    count_jobs(s, all);
-    const uint32_t total = min(all, b.job_cap);
-    const bool prefix = prefix_mode(mode);
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (uint32_t base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
-        const uint32_t t = base + threadIdx.x;
-        int req = kReqDone;
-        if (t < total) {
-            ShiftJob j;
-            j.code = b.job_items[t];
-            Hit dh;
-            const ShiftSrc src = resolve_job(fp, b, mode, j.code, &dh);
-            const Isect cur = job_dst(s, mode, dh);
+struct ShiftLane {
+    uint32_t phase, code, left;  // left: replays to go
+    V3 o, d;                     // the ray in flight
+    float tmax;                  // shadow ray: the edge's length
+    float4 acc;                  // replays: throughput; shadow ray: the result if the edge is visible
+    Rng rng;                     // the source path's replay
+
+    RT_D void start(uint32_t job_code) {
+        code = job_code;
+        phase = kJobStart;
+    }
+    RT_D void finish(const Bufs& b, float4 v) {
+        job_out(b, code, v);
+        phase = kJobDone;
+    }
+
+    RT_D void step(const SceneView& s, const FrameParams& fp, const Bufs& b, int mode, const TraceResult& h) {
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (phase == kJobShadow) {
+            finish(b, h.prim != CRISB_INVALID_PRIM ? zero : acc);
+            return;
+        }
+        const bool prefix = prefix_mode(mode), fresh = phase == kJobStart;
+        Isect cur;
+        V3 tp = splat(1.0f);
+        if (!fresh) {
+            hit_isect(s, h, d, cur);
+            if (!cur.valid) {
+                finish(b, zero);
+                return;
+            }
+            tp = V3{acc.x, acc.y, acc.z};
+        }
+        Hit dh;
+        const ShiftSrc src = resolve_job(fp, b, mode, code, fresh ? &dh : nullptr);
+        if (fresh) {
+            cur = job_dst(s, mode, dh);
             bool ok = fl_valid(src.flags) && cur.valid;
             if (prefix) ok = ok && fl_recon(src.flags) >= 2;
             ok = ok && unpack(s, src.anchor).valid && unpack(s, src.recon).valid;
             if (!ok) {
-                job_out(b, j.code, zero);
-            } else {
-                const int skip = prefix ? 2 : 1;
-                const uint32_t left = static_cast<uint32_t>(max(static_cast<int>(fl_recon(src.flags)) - skip, 0));
-                Rng srng{src.rng};
-                req = shift_advance<kTex>(s, b, prefix, src, j, cur, srng, splat(1.0f), left, false);
-                if (req != kReqDone) job_store(b.jobs + t, j);
+                finish(b, zero);
+                return;
+            }
+            left = static_cast<uint32_t>(max(static_cast<int>(fl_recon(src.flags)) - (prefix ? 2 : 1), 0));
+            rng = Rng{src.rng};
+        }
+        if (left > 0) {
+            rng.next_float();
+            const BrdfSample bs = brdf_sample<kTex>(s, cur, rng);
+            if (bs.pdf <= 0.0f) {
+                finish(b, zero);
+                return;
+            }
+            tp = tp * bs.brdf;
+            --left;
+            o = cur.pos;
+            d = bs.dir;
+            acc = f4(tp, 0.0f);
+            phase = kJobHit;
+            return;
+        }
+        // the reconnection edge
+        const Isect src_anchor = unpack(s, src.anchor);
+        Isect src_recon = unpack(s, src.recon);
+        const V3 rv = src_recon.pos - cur.pos;
+        const float rlen = length(rv);
+        const V3 rdir = normalize(rv);
+        if ((prefix && isinf(rlen)) || nonfinite(rdir)) {
+            finish(b, zero);
+            return;
+        }
+        const BrdfEval b1 = brdf_eval<kTex>(s, cur, rdir);
+        float4 res = zero;
+        if (b1.pdf > 0.0f) {
+            tp = tp * b1.brdf;
+            bool ok = true;
+            if (prefix || fl_recon(src.flags) < fl_len(src.flags)) {
+                src_recon.dir = rdir;
+                if (!prefix && is_zero(src.rod)) ok = false;
+                if (ok) {
+                    const BrdfEval b2 = brdf_eval<kTex>(s, src_recon, src.rod);
+                    if (b2.pdf <= 0.0f) ok = false;
+                    else tp = tp * b2.brdf;
+                }
+            }
+            if (ok) {
+                const float jac = recon_jacobian(src_anchor.pos, cur.pos, src_recon.pos, src_recon.nrm);
+                const V3 f = prefix ? gmax(splat(0.0f), tp * src.prf) : tp * src.prf;
+                res = f4(f, jac);
             }
         }
-        job_push(b, 0, req, t);
-    }
-}
-
-// list entries beyond the machines' capacity: the same job, every ray traced
-// in place (shift_advance with inline rays is the machine's own step)
-template <bool kTex>
-__global__ void __launch_bounds__(kPassBlock) k_shift_overflow(SceneView s, FrameParams fp, Bufs b, int mode) {
-    const uint32_t total = *b.job_count;
-    const bool prefix = prefix_mode(mode);
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (uint32_t t = b.job_cap + blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        ShiftJob j;
-        j.code = b.job_items[t];
-        Hit dh;
-        const ShiftSrc src = resolve_job(fp, b, mode, j.code, &dh);
-        const Isect cur = job_dst(s, mode, dh);
-        bool ok = fl_valid(src.flags) && cur.valid;
-        if (prefix) ok = ok && fl_recon(src.flags) >= 2;
-        ok = ok && unpack(s, src.anchor).valid && unpack(s, src.recon).valid;
-        if (!ok) {
-            job_out(b, j.code, zero);
-            continue;
+        if ((__float_as_uint(res.x) | __float_as_uint(res.y) | __float_as_uint(res.z) | __float_as_uint(res.w)) ==
+            0u) {
+            finish(b, zero);  // +0 whether or not the edge is visible
+            return;
         }
-        const int skip = prefix ? 2 : 1;
-        const uint32_t left = static_cast<uint32_t>(max(static_cast<int>(fl_recon(src.flags)) - skip, 0));
-        Rng srng{src.rng};
-        shift_advance<kTex>(s, b, prefix, src, j, cur, srng, splat(1.0f), left, true);
+        o = cur.pos;
+        d = rdir;
+        tmax = rlen;
+        acc = res;
+        phase = kJobShadow;
+    }
+
+    // a job waiting for its ray between launches: everything but the hit word,
+    // which the traversal kernels write
+    RT_D void save(ShiftJob* r) const {
+        r->o = f4(o, tmax);
+        r->d = f4(d, 0.0f);
+        r->acc = acc;
+        r->rng = rng.state;
+        r->code = code;
+        r->ctr = left;
+    }
+    RT_D void load(const ShiftJob* r, bool shadow) {
+        phase = shadow ? kJobShadow : kJobHit;
+        const float4 a = r->o, c = r->d;
+        o = V3{a.x, a.y, a.z};
+        tmax = a.w;
+        d = V3{c.x, c.y, c.z};
+        acc = r->acc;
+        rng.state = r->rng;
+        code = r->code;
+        left = r->ctr;
+    }
+    // the traced ray's result (set_hit, set_occluded)
+    RT_D static TraceResult result(const ShiftJob* r, bool shadow) {
+        const float4 h = r->hit;
+        if (shadow) return TraceResult{__float_as_uint(h.x) ? 0u : CRISB_INVALID_PRIM, 0.0f, 0.0f, 0.0f};
+        return TraceResult{__float_as_uint(h.x), h.y, h.z, h.w};
+    }
+};
+
+// first step of the list's jobs (as many as the machines have records for); 8
+// resident blocks per SM, 6 and 7 within 1%
+template <bool kTex>
+__global__ void __launch_bounds__(kPassBlock, 8) k_shift_begin(SceneView s, FrameParams fp, Bufs b, int mode) {
+    const uint32_t all = *b.job_count;
+    count_jobs(s, all);
+    const uint32_t total = min(all, b.job_cap);
+    for (uint32_t base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
+        const uint32_t t = base + threadIdx.x;
+        ShiftLane<kTex> job;
+        job.phase = kJobDone;
+        if (t < total) {
+            job.start(b.job_items[t]);
+            job.step(s, fp, b, mode, TraceResult{});
+            if (job.phase != kJobDone) job.save(b.jobs + t);
+        }
+        job_push(b, 0, job.phase, t);
     }
 }
 
-// resume every job whose ray of round `round` finished; in the last round jobs
-// with replays left finish inline
-template <bool kLast, bool kTex>
-__global__ void __launch_bounds__(kPassBlock) k_shift_step(SceneView s, FrameParams fp, Bufs b, int mode, int round) {
-    const uint32_t nc = b.job_qcount[2 * round], ns = b.job_qcount[2 * round + 1];
-    const uint32_t total = nc + ns;
+// takes the result of every ray of round `round` to its job's next ray, queued for
+// the next round, or its end
+template <bool kTex>
+__global__ void __launch_bounds__(kPassBlock, 8) k_shift_step(SceneView s, FrameParams fp, Bufs b, int mode, int round) {
+    const uint32_t nc = b.job_qcount[2 * round], total = nc + b.job_qcount[2 * round + 1];
     const uint32_t* qc = b.job_queue[2 * (round & 1)];
     const uint32_t* qs = b.job_queue[2 * (round & 1) + 1];
-    const bool prefix = prefix_mode(mode);
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (uint32_t base = blockIdx.x * blockDim.x; base < total; base += gridDim.x * blockDim.x) {
         const uint32_t u = base + threadIdx.x;
-        int req = kReqDone;
+        ShiftLane<kTex> job;
+        job.phase = kJobDone;
         uint32_t t = 0;
         if (u < total) {
             t = u < nc ? qc[u] : qs[u - nc];
-            const ShiftJob* jr = b.jobs + t;
-            if (u >= nc) {
-                // the shadow ray's result: occluded flag, prepared value, job code
-                job_out(b, jr->code, __float_as_uint(jr->hit.x) ? zero : jr->acc);
-            } else {
-                ShiftJob j;  // o is written before it is read
-                j.d = jr->d;
-                j.hit = jr->hit;
-                j.acc = jr->acc;
-                j.rng = jr->rng;
-                j.code = jr->code;
-                j.ctr = jr->ctr;
-                // trace_closest semantics: interpolated, normalised normal
-                Isect it;
-                const uint32_t prim = __float_as_uint(j.hit.x);
-                it.dir = f3(j.d);
-                it.valid = prim != CRISB_INVALID_PRIM;
-                if (!it.valid) {
-                    job_out(b, j.code, zero);
-                } else {
-                    it.prim = prim;
-                    it.bu = j.hit.z;
-                    it.bv = j.hit.w;
-                    const ShadeTri tri = load_shade(s, prim);
-                    it.pos = interp(it.bu, it.bv, tri.p0, tri.p1, tri.p2);
-                    it.nrm = normalize(interp(it.bu, it.bv, tri.n0, tri.n1, tri.n2));
-                    const ShiftSrc src = resolve_job(fp, b, mode, j.code, nullptr);
-                    Rng srng{j.rng};
-                    req = shift_advance<kTex>(s, b, prefix, src, j, it, srng, f3(j.acc), j.ctr, kLast);
-                    if (req != kReqDone) job_store(b.jobs + t, j);
+            job.load(b.jobs + t, u >= nc);
+            job.step(s, fp, b, mode, ShiftLane<kTex>::result(b.jobs + t, u >= nc));
+            if (job.phase != kJobDone) job.save(b.jobs + t);
+        }
+        job_push(b, round + 1, job.phase, t);
+    }
+}
+
+// The jobs on persistent warps, as the path flows (wavefront.cu): the whole list
+// (round < 0), or the jobs whose rays round `round` traced and the list's entries
+// beyond the machines' records.
+template <bool kTex>
+__global__ void __launch_bounds__(kPassBlock, 5) k_shift(SceneView s, FrameParams fp, Bufs b, int mode, int round) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const uint32_t all = *b.job_count;
+    uint32_t nc = 0, nq = 0, first = 0;  // queued jobs, and the first list entry started here
+    const uint32_t* qc = nullptr;
+    const uint32_t* qs = nullptr;
+    if (round < 0) {
+        count_jobs(s, all);
+    } else {
+        nc = b.job_qcount[2 * round];
+        nq = nc + b.job_qcount[2 * round + 1];
+        qc = b.job_queue[2 * (round & 1)];
+        qs = b.job_queue[2 * (round & 1) + 1];
+        first = min(all, b.job_cap);
+    }
+    WorkPool pool(nq + (all - first), b.job_next);
+    ShiftLane<kTex> job;
+    job.phase = kJobDone;
+    bool traced = false;  // the lane's ray has its result in h
+    TraceResult h{CRISB_INVALID_PRIM, 0.0f, 0.0f, 0.0f};
+    while (true) {
+        while (true) {
+            if (traced || job.phase == kJobStart) {
+                job.step(s, fp, b, mode, h);
+                traced = false;
+            }
+            if (pool.more()) {
+                const bool want = job.phase == kJobDone;
+                if (__any_sync(kFull, want)) {
+                    const uint32_t u = pool.take(want);
+                    if (u != 0xffffffffu) {
+                        if (u < nq) {
+                            const uint32_t t = u < nc ? qc[u] : qs[u - nc];
+                            job.load(b.jobs + t, u >= nc);
+                            h = ShiftLane<kTex>::result(b.jobs + t, u >= nc);
+                            traced = true;
+                        } else {
+                            job.start(b.job_items[first + (u - nq)]);
+                        }
+                    }
                 }
             }
+            const unsigned lacking =
+                __ballot_sync(kFull, traced || job.phase == kJobStart || (job.phase == kJobDone && pool.more()));
+            if (!lacking) break;
+            if (__popc(lacking) <= kMostIdle && __any_sync(kFull, !traced && job.phase > kJobStart)) break;
         }
-        if (!kLast) job_push(b, round + 1, req, t);
+        if (!__any_sync(kFull, job.phase != kJobDone)) break;
+        if (!traced && job.phase > kJobStart) {
+            const bool shadow = job.phase == kJobShadow;
+            count_ray(s, shadow ? 1 : 0);
+            h = traverse_ray(s, job.o, job.d, 1e-3f, shadow ? job.tmax : 1e16f, shadow);
+            traced = true;
+        }
     }
 }
 
@@ -1132,7 +1167,7 @@ unsigned path_tracer_grid() {
 }
 
 struct ShiftGrids {
-    unsigned begin, step, step_last, overflow;
+    unsigned begin, step, persistent;
 };
 
 template <bool kTex>
@@ -1141,9 +1176,8 @@ const ShiftGrids& shift_grids() {
     static ShiftGrids g{};
     std::call_once(once, [] {
         g.begin = persistent_grid(reinterpret_cast<const void*>(k_shift_begin<kTex>));
-        g.step = persistent_grid(reinterpret_cast<const void*>(k_shift_step<false, kTex>));
-        g.step_last = persistent_grid(reinterpret_cast<const void*>(k_shift_step<true, kTex>));
-        g.overflow = persistent_grid(reinterpret_cast<const void*>(k_shift_overflow<kTex>));
+        g.step = persistent_grid(reinterpret_cast<const void*>(k_shift_step<kTex>));
+        g.persistent = persistent_grid(reinterpret_cast<const void*>(k_shift<kTex>));
     });
     return g;
 }
@@ -1154,48 +1188,52 @@ const ShiftGrids& shift_grids() {
         if (m) m->mark(cls, st); \
     } while (0)
 
-// Rounds of a shift phase: at most kShiftRounds, fewer where the jobs trace
-// fewer rays.  A prefix shift replays the vertices before its reconnection
-// vertex but the first two (none for a prefix of length 2) and then tests the
-// edge.  At least one: a reservoir kept from a frame with another prefix length
-// may need more rays, which the last round's step traces in place.
-int shift_rounds(const crisb_params& p, int mode) {
-    if (!prefix_mode(mode)) return kShiftRounds;
-    const int len = p.renderer_type == CRISB_RENDERER_CONDITIONAL_RESTIR ? p.prefix_len : p.max_path_len;
-    return std::min(std::max(len - 1, 1), kShiftRounds);
+// Rounds before the persistent kernel (see flow_rounds): most jobs trace one or
+// two rays, so the rays of one round fill the GPU and those left do not.  None to
+// 512x384 (RestirPt frames of the room 0.87 ms against 1.01 with one, conditional
+// ones 2.29 against 2.35; at 641x479 textured jobs that replay long prefixes, two
+// to a lane, take 1.17 against 0.67), one above (960x540 4.45 ms against 4.54 with
+// none, 4.74 with two, 4.91 with three; 1080p 14.0 against 15.0, 14.0, 14.3), two
+// for views that render beside one another (16 views: 76.0 ms, 78.3 with one).
+// Three rounds whose last step traced the rays left in place, a thread a job, took
+// 4.95 and 14.3 ms.
+int shift_rounds(const FrameParams& fp) {
+    if (fp.concurrent) return 2;
+    return fp.width * fp.height <= 196608u ? 0 : 1;
 }
 
 // the counters of one path flow and one shift phase
 void take_counters(Bufs& b, Counters& c) {
-    uint32_t* p = c.take(2 * (kMaxFlowRounds + 1) + 2 + 2 * kShiftRounds);
+    uint32_t* p = c.take(2 * (kMaxFlowRounds + 1) + 3 + 2 * (kMaxShiftRounds + 1));
     b.path_counts = p;
     b.path_next = p + 2 * (kMaxFlowRounds + 1);
     b.job_count = b.path_next + 1;
-    b.job_qcount = b.job_count + 1;
+    b.job_next = b.path_next + 2;
+    b.job_qcount = b.path_next + 3;
 }
 
-// the shift jobs of the list: begin, then rounds of trace / step
+// the shift jobs of the list: rounds of trace / step, then persistent warps
 template <bool kTex>
 void run_shift_jobs_as(const SceneView& s, const FrameParams& fp, const Bufs& b, int mode, cudaStream_t st,
                        Marker* m) {
     const ShiftGrids& g = shift_grids<kTex>();
-    const int rounds = shift_rounds(fp.p, mode);
-    k_shift_begin<kTex><<<g.begin, kPassBlock, 0, st>>>(s, fp, b, mode);
-    MARK(kClsShift);
-    k_shift_overflow<kTex><<<g.overflow, kPassBlock, 0, st>>>(s, fp, b, mode);
-    MARK(kClsShift);
+    const int rounds = shift_rounds(fp);
+    if (rounds > 0) {
+        k_shift_begin<kTex><<<g.begin, kPassBlock, 0, st>>>(s, fp, b, mode);
+        MARK(kClsShift);
+    }
     for (int r = 0; r < rounds; ++r) {
         const int q = 2 * (r & 1);
         launch_trace<ShiftJob>(fp.trace_block, fp.trace_grid, b.job_cap, st, s, b.job_queue[q], b.job_qcount + 2 * r,
                                b.job_queue[q + 1], b.job_qcount + 2 * r + 1, b.jobs);
         MARK(kClsTrace);
         if (r + 1 < rounds) {
-            k_shift_step<false, kTex><<<g.step, kPassBlock, 0, st>>>(s, fp, b, mode, r);
-        } else {
-            k_shift_step<true, kTex><<<g.step_last, kPassBlock, 0, st>>>(s, fp, b, mode, r);
+            k_shift_step<kTex><<<g.step, kPassBlock, 0, st>>>(s, fp, b, mode, r);
+            MARK(kClsShift);
         }
-        MARK(kClsShift);
     }
+    k_shift<kTex><<<g.persistent, kPassBlock, 0, st>>>(s, fp, b, mode, rounds - 1);
+    MARK(kClsShift);
 }
 
 // the shift kernels come in two builds: with the texture lookup, for scenes
@@ -1211,9 +1249,7 @@ void run_shift_jobs(const SceneView& s0, const FrameParams& fp, const Bufs& b, i
 
 }  // namespace
 
-uint32_t shift_launches(const crisb_params& p, int mode) {
-    return 2 + 2 * static_cast<uint32_t>(shift_rounds(p, mode));
-}
+uint32_t shift_launches(const FrameParams& fp) { return 1 + 2 * static_cast<uint32_t>(shift_rounds(fp)); }
 
 void launch_prefix_gen_temp_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                   cudaStream_t st, Marker* m) {

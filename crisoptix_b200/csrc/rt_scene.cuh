@@ -183,11 +183,16 @@ RT_D void dev_error(const SceneView& s, int code) {
     if (s.err) atomicOr(s.err, code);
 }
 
-// statistics: one warp-aggregated atomic per call site
+// statistics: warp-aggregated atomics, one per kind of ray among the lanes
 RT_D void count_ray(const SceneView& s, int which) {
     if (!s.ray_count) return;
     const unsigned m = __activemask();
-    if ((threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(&s.ray_count[which], static_cast<unsigned long long>(__popc(m)));
+    const unsigned one = __ballot_sync(m, which == 1), zero = m & ~one;
+    const unsigned lane = threadIdx.x & 31u;
+    if (zero && lane == static_cast<unsigned>(__ffs(zero) - 1))
+        atomicAdd(&s.ray_count[0], static_cast<unsigned long long>(__popc(zero)));
+    if (one && lane == static_cast<unsigned>(__ffs(one) - 1))
+        atomicAdd(&s.ray_count[1], static_cast<unsigned long long>(__popc(one)));
 }
 
 // Traversal of one ray as a resumable state: step() visits one node (both

@@ -77,11 +77,6 @@ __global__ void __launch_bounds__(kPassBlock, 5) k_flow_shade(SceneView s, Frame
 // side in one traversal), steps, and takes another path when it has ended:
 // every pixel's path from its start (round < 0), or the paths whose rays are
 // queued for round `round`.
-// lanes that may go without a ray into a traversal rather than have the others
-// wait for one more step (0 / 4 / 8 / 16 / 24: 14.79, 14.64, 14.57, 14.70, 14.86 ms per
-// 1080p frame with one more round a flow than now)
-constexpr int kMostIdle = 8;
-
 template <int kFlow, bool kTex>
 __global__ void __launch_bounds__(kPassBlock, 5) k_flow(SceneView s, FrameParams fp, Bufs b, int round) {
     constexpr unsigned kFull = 0xffffffffu;

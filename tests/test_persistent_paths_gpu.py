@@ -42,3 +42,24 @@ def test_frozen_path_tracer_is_the_path_tracer(cuda_device, w, h):
     g2, e2 = adj.gradient([cam], 2.0 * ones)
     np.testing.assert_allclose(2.0 * e1.cpu().numpy(), e2.cpu().numpy(), rtol=1e-4, atol=1e-6)
     np.testing.assert_allclose(2.0 * g1.cpu().numpy(), g2.cpu().numpy(), rtol=1e-3, atol=1e-4)
+
+
+@pytest.mark.parametrize("nee", [0.0, 1.0])
+def test_ray_counts_by_kind(cuda_device, nee):
+    """Lanes that trace a closest-hit and a shadow ray side by side count each as
+    what it is: with NEE at every vertex a path is one closest-hit ray and at most
+    one shadow ray, without NEE it traces no shadow ray."""
+    from crisoptix_b200 import Renderer
+
+    desc, cam = scenes.cornell_box()
+    sc = Scene(desc)
+    w, h = 97, 53
+    r = Renderer(w, h, sc, default_params(sc.scene_size, renderer_type=_abi.PATH_TRACER, max_path_len=4, nee_prob=nee))
+    r.set_timing(2)
+    r.launch_frame(cam, torch.zeros(h, w, 3, device="cuda").data_ptr())
+    torch.cuda.synchronize()
+    st = r.stats()
+    if nee == 1.0:
+        assert st["closest_rays"] == w * h and 0 < st["shadow_rays"] <= w * h
+    else:
+        assert st["closest_rays"] > w * h and st["shadow_rays"] == 0
