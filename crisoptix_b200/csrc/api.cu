@@ -1024,7 +1024,7 @@ struct crisb_renderer {
 
     void tonemap_epilogue(const float* out, cudaStream_t st, Marker* m) {
         if (!srgb_out) return;
-        check(launch_tonemap_srgb8(out, srgb_out, width * height, st), "tonemap");
+        check(launch_tonemap_srgb8(out, srgb_out, width * height, st, false), "tonemap");
         if (m) m->mark(kClsOther, st);
         ++launches;
     }
@@ -1525,7 +1525,7 @@ int crisb_tonemap_srgb8(const float* rgb_dev, uint8_t* srgb_dev, uint32_t num_pi
     return guarded([&] {
         if (num_pixels == 0) return;  // nothing is read or written
         require(rgb_dev && srgb_dev, "null argument");
-        check(launch_tonemap_srgb8(rgb_dev, srgb_dev, num_pixels, static_cast<cudaStream_t>(stream)), "tonemap");
+        check(launch_tonemap_srgb8(rgb_dev, srgb_dev, num_pixels, static_cast<cudaStream_t>(stream), true), "tonemap");
     });
 }
 

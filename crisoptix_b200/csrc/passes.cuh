@@ -219,8 +219,9 @@ void restir_adjoint_backward(const SceneView& eval, const crisb_material* frame_
                              const crisb_emitter* frame_emitters, uint32_t num_mats, const FrameParams& fp,
                              const Bufs& b, float4* pairs, const float* d_img, float* g_mat, float* g_em,
                              cudaStream_t st);
-// sRGB tone mapping of n float RGB pixels to bytes (tonemap.cu)
-cudaError_t launch_tonemap_srgb8(const float* rgb, uint8_t* out, uint32_t n, cudaStream_t st);
+// sRGB tone mapping of n float RGB pixels to bytes (tonemap.cu); `beside`: the
+// launch may start beside the end of the stream's work before it
+cudaError_t launch_tonemap_srgb8(const float* rgb, uint8_t* out, uint32_t n, cudaStream_t st, bool beside);
 // the kernel's step table: t256[k] smallest float with byte >= k, and c_max
 void srgb8_thresholds(float* t256, float* c_max);
 // generic LBVH stages over `cap` primitives (count in w.n)
