@@ -27,7 +27,7 @@ cudaError_t sort_high32(const uint64_t* keys_in, uint64_t* keys_out, void* temp,
                         cudaStream_t st);
 
 // launches one sort_high32 enqueues
-constexpr uint32_t kLaunches = 20;
+constexpr uint32_t kLaunches = 16;
 
 // Exclusive prefix sum of n uint32 values (in and out may alias); the grand
 // total to *total (device memory) when total is not null.  `temp` holds
