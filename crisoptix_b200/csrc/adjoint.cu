@@ -238,24 +238,6 @@ __global__ void __launch_bounds__(kPassBlock, 6) k_frozen_forward(AdjView a, Fra
 constexpr uint32_t kGroup = 128;
 constexpr int kGroupThreads = 64;
 
-// the pixels of a block's group, taken by its lanes in turn
-struct GroupPool {
-    uint32_t first, count;
-    uint32_t* taken;  // shared
-    RT_D bool more() const {
-        const uint32_t t = __shfl_sync(0xffffffffu, *static_cast<volatile uint32_t*>(taken), 0);
-        return t < count;
-    }
-    RT_D uint32_t take(bool want) {
-        const unsigned m = __ballot_sync(0xffffffffu, want);
-        const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
-        uint32_t v = 0;
-        if (lane == leader) v = atomicAdd(taken, static_cast<uint32_t>(__popc(m)));
-        v = __shfl_sync(0xffffffffu, v, leader) + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
-        return want && v < count ? first + v : 0xffffffffu;
-    }
-};
-
 __global__ void __launch_bounds__(kGroupThreads, 10) k_frozen_backward(AdjView a, FrameParams fp, const float* d_img,
                                                                       float* g_mat, float* g_em, int use_shared) {
     extern __shared__ float sh[];
@@ -306,8 +288,9 @@ void adjoint_backward(const SceneView& eval, const crisb_material* sample_mats, 
     const AdjView a{eval, sample_mats, num_mats, eval.num_emitters};
     const uint32_t P = fp.width * fp.height;
     const size_t sh_bytes = (static_cast<size_t>(num_mats) * kMatGrad + eval.num_emitters * kEmGrad) * sizeof(float);
-    const int use_shared = sh_bytes <= 48u * 1024u ? 1 : 0;
+    const int use_shared = sh_bytes <= kSharedGradBytes ? 1 : 0;
     const size_t shb = use_shared ? sh_bytes : 0;
+    allow_shared_grads(reinterpret_cast<const void*>(k_frozen_backward), shb);
     k_frozen_backward<<<(P + kGroup - 1) / kGroup, kGroupThreads, shb, st>>>(a, fp, d_img, g_mat, g_em, use_shared);
 }
 

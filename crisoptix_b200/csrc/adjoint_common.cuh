@@ -103,5 +103,33 @@ struct GradSink {
     }
 };
 
+// the items [first, first + count) of a block, taken by its lanes in turn
+struct GroupPool {
+    uint32_t first, count;
+    uint32_t* taken;  // shared
+    RT_D bool more() const {
+        const uint32_t t = __shfl_sync(0xffffffffu, *static_cast<volatile uint32_t*>(taken), 0);
+        return t < count;
+    }
+    RT_D uint32_t take(bool want) {
+        const unsigned m = __ballot_sync(0xffffffffu, want);
+        const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+        uint32_t v = 0;
+        if (lane == leader) v = atomicAdd(taken, static_cast<uint32_t>(__popc(m)));
+        v = __shfl_sync(0xffffffffu, v, leader) + static_cast<uint32_t>(__popc(m & ((1u << lane) - 1u)));
+        return want && v < count ? first + v : 0xffffffffu;
+    }
+};
+
+// Parameter blocks of up to 48 KB are gathered in shared memory, beside what the
+// kernel itself declares there; together that may pass the 48 KB a launch gets
+// without asking.
+constexpr size_t kSharedGradBytes = 48u * 1024u;
+
+inline void allow_shared_grads(const void* kernel, size_t bytes) {
+    if (bytes + 4096u > kSharedGradBytes)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSharedGradBytes));
+}
+
 }  // namespace
 }  // namespace crisb

@@ -184,23 +184,34 @@ RT_D void seg_prefix(const RAdjView& a, const FrameParams& fp, const Prefix& cp,
     }
 }
 
-// Fs: TraceSuffix of a valid gather suffix (path_gen.h:252-387)
+// Fs: TraceSuffix of a valid gather suffix (path_gen.h:252-387), a vertex a step,
+// so that a lane can go on with the next pixel's where its own ends
 template <bool kGrad>
-RT_D void seg_suffix(const RAdjView& a, const FrameParams& fp, const Suffix& cs, Seg<kGrad>& sg) {
-    sg.init();
-    Rng rng{cs.rng};
-    const float nee = fp.p.nee_prob;
-    const uint32_t max_len = static_cast<uint32_t>(fp.p.max_path_len - fp.p.prefix_len);
-    Isect it = unpack(a.eval, cs.last_prefix);
-    V3 last_dir = splat(0.0f);
-    for (uint32_t vi = 0; vi < max_len; ++vi) {
+struct SuffixPath {
+    Seg<kGrad> sg;
+    Rng rng;
+    Isect it;
+    V3 dir;
+    uint32_t vi;
+
+    RT_D void begin(const RAdjView& a, const Suffix& cs) {
+        sg.init();
+        rng = Rng{cs.rng};
+        it = unpack(a.eval, cs.last_prefix);
+        dir = splat(0.0f);
+        vi = 0;
+    }
+    // false: the path has ended and sg is complete
+    RT_D bool step(const RAdjView& a, const FrameParams& fp) {
+        const uint32_t max_len = static_cast<uint32_t>(fp.p.max_path_len - fp.p.prefix_len);
+        if (vi >= max_len) return false;
         if (vi > 0) {
-            const V3 last_pos = it.pos;
-            trace_closest(a.eval, last_pos, last_dir, 1e-3f, 1e16f, it);
-            if (!it.valid) return;
+            const V3 pos = it.pos;
+            trace_closest(a.eval, pos, dir, 1e-3f, 1e16f, it);
+            if (!it.valid) return false;
         }
         const bool force_nee = vi == max_len - 1;
-        if (rng.next_float() < nee || force_nee) {
+        if (rng.next_float() < fp.p.nee_prob || force_nee) {
             const EmitterSample es = sample_emitter(a.eval, rng);
             const V3 light_vec = es.pos - it.pos;
             const float light_len = length(light_vec);
@@ -208,14 +219,16 @@ RT_D void seg_suffix(const RAdjView& a, const FrameParams& fp, const Suffix& cs,
             uint32_t mi;
             const BrdfGrad g = grad_at(a, it, light_dir, mi);
             mul_nee(sg, g, mi, es, 1.0f / (light_len * light_len));
-            return;
+            return false;
         }
         const BrdfSample bs = brdf_sample(a.samp, it, rng);
         uint32_t mi;
         sg.mul_brdf(grad_at(a, it, bs.dir, mi), mi);
-        last_dir = bs.dir;
+        dir = bs.dir;
+        ++vi;
+        return true;
     }
-}
+};
 
 // T_n: the throughput of the shift of `src` onto the vertex `dst_last`
 // (suffix CalcCurrContribInOtherDomain, suffix_reuse.h:10-108) before its
@@ -355,68 +368,84 @@ RT_D NeighTerm neigh_term(const FrameParams& fp, const Bufs& b, uint32_t i, uint
     return t;
 }
 
-// One pixel: kGrad false returns the frozen estimator's value at theta, its
-// neighbour terms read from `pairs`; kGrad true adds dl . dL/dtheta of the
-// canonical factors at theta0 to the sink, writes the neighbour terms'
-// weights into `pairs` and returns zero.
+// What a pixel's canonical suffix, replayed after the rest of it, goes into.
 template <bool kGrad>
-RT_D V3 gather_pixel(const RAdjView& a, const FrameParams& fp, const Bufs& b, uint32_t i, V3 dl, GradSink* sink,
-                     float4* pairs) {
-    if (b.canon_prefix[i].primary.prim == CRISB_INVALID_PRIM) return splat(0.0f);  // no gather ran
+struct SuffixItem;
+template <>
+struct SuffixItem<true> {
+    uint32_t pixel;
+    V3 w;  // dLoss / dFs
+};
+template <>
+struct SuffixItem<false> {
+    uint32_t pixel;
+    V3 fpv, gather;  // Fp at theta; the neighbours' part of the pixel
+    float pq, canon_mis, d;
+    RT_D V3 pixel_value(V3 fs) const {
+        const V3 canon = fpv * fs / pq;
+        return d == 0.0f ? canon : (gather + (canon * canon_mis)) / d;
+    }
+};
+
+// One pixel up to its canonical suffix: true fills `item` with what that goes
+// into, false leaves the pixel's value in `value`.  kGrad false: the frozen
+// estimator at theta, its neighbour terms read from `pairs`; kGrad true adds
+// dl . dL/dtheta of the canonical prefix at theta0 to the sink and writes the
+// neighbour terms' weights into `pairs`.
+template <bool kGrad>
+RT_D bool gather_pixel(const RAdjView& a, const FrameParams& fp, const Bufs& b, uint32_t i, V3 dl, GradSink* sink,
+                       float4* pairs, V3& value, SuffixItem<kGrad>& item) {
+    value = splat(0.0f);
+    if (b.canon_prefix[i].primary.prim == CRISB_INVALID_PRIM) return false;  // no gather ran
     const Prefix cp = ld_prefix_v(b.gather_cp[i]);
-    if (!fl_valid(cp.flags)) return splat(0.0f);
+    if (!fl_valid(cp.flags)) return false;
     Seg<kGrad> sg;
     if (fl_nee(cp.flags)) {  // the gather prefix ended in NEE: Fp / Pp
-        if (kGrad && nonfinite(cp.f / cp.p)) return splat(0.0f);
+        if (kGrad && nonfinite(cp.f / cp.p)) return false;
         seg_prefix(a, fp, cp, sg);
         sg.emit(dl / cp.p, sink);
-        return sg.val / cp.p;
+        value = sg.val / cp.p;
+        return false;
     }
     const Suffix cs = ld_suffix(b.gather_cs[i].sample);
-    if (!fl_valid(cs.flags)) return splat(0.0f);
+    if (!fl_valid(cs.flags)) return false;
     const float pp = cp.p, ps = cs.p;
-    if (fp.k == 0) {  // canonical contribution alone: Fp Fs / (Pp Ps)
-        if (kGrad) {
-            if (nonfinite(cp.f * cs.f / (pp * ps))) return splat(0.0f);
-            seg_prefix(a, fp, cp, sg);
-            sg.emit(dl * cs.f / (pp * ps), sink);
-            seg_suffix(a, fp, cs, sg);
-            sg.emit(dl * cp.f / (pp * ps), sink);
-            return splat(0.0f);
-        }
-        seg_prefix(a, fp, cp, sg);
-        const V3 fpv = sg.val;
-        seg_suffix(a, fp, cs, sg);
-        return fpv * sg.val / (pp * ps);
-    }
-    // the frozen weights, from what k_gather_combine read
+    item.pixel = i;
+    // the frozen weights, from what k_gather_combine read; fp.k == 0: the
+    // canonical contribution alone, Fp Fs / (Pp Ps)
     const uint32_t P = pixel_count(fp);
-    const uint32_t count = b.neigh_count[i];
-    const uint32_t vflags = b.pass_flags[i];
+    const uint32_t count = fp.k > 0 ? b.neigh_count[i] : 0;
+    const uint32_t vflags = fp.k > 0 ? b.pass_flags[i] : 0;
     const uint32_t nvalid = __popc(vflags);
     const float K = static_cast<float>(nvalid);
     const float E = static_cast<float>(nvalid + 1), D = K + 1.0f;
-    const float4* sh = b.shift_out + static_cast<size_t>(i) * b.slots;
     V3 s0 = splat(0.0f);
     float canon_mis = 1.0f;
-    for (uint32_t n = 0; n < count; ++n) {
-        if (!(vflags & (1u << n))) continue;
-        const NeighTerm t = neigh_term(fp, b, i, n, K);
-        if (t.used) s0 = s0 + t.nmis * t.f0 * t.nwsum * t.jac;
-        const float4 o1 = sh[2 * n + 1];
-        canon_mis += mis_canonical(cs.f, xyz(o1), o1.w, K, 1.0f, sres_conf(b.sres_cur, t.np));
-    }
-    {
+    if (fp.k == 0) {
+        if (kGrad && nonfinite(cp.f * cs.f / (pp * ps))) return false;
+    } else {
+        const float4* sh = b.shift_out + static_cast<size_t>(i) * b.slots;
+        for (uint32_t n = 0; n < count; ++n) {
+            if (!(vflags & (1u << n))) continue;
+            const NeighTerm t = neigh_term(fp, b, i, n, K);
+            if (t.used) s0 = s0 + t.nmis * t.f0 * t.nwsum * t.jac;
+            const float4 o1 = sh[2 * n + 1];
+            canon_mis += mis_canonical(cs.f, xyz(o1), o1.w, K, 1.0f, sres_conf(b.sres_cur, t.np));
+        }
         V3 g0 = s0 * cp.f / pp;
         g0 = g0 / E;
         const V3 r0 = (g0 + (cp.f * cs.f / (pp * ps)) * canon_mis) / D;
-        if (nonfinite(r0)) return splat(0.0f);  // the frame stored zero
+        if (nonfinite(r0)) return false;  // the frame stored zero
     }
-    if (kGrad) {
-        seg_prefix(a, fp, cp, sg);
+    seg_prefix(a, fp, cp, sg);
+    if constexpr (kGrad) {
+        if (fp.k == 0) {
+            sg.emit(dl * cs.f / (pp * ps), sink);
+            item.w = dl * cp.f / (pp * ps);
+            return true;
+        }
         sg.emit(dl * ((s0 / pp) / E + (cs.f / (pp * ps)) * canon_mis) / D, sink);
-        seg_suffix(a, fp, cs, sg);
-        sg.emit(dl * (cp.f / (pp * ps)) * canon_mis / D, sink);
+        item.w = dl * (cp.f / (pp * ps)) * canon_mis / D;
         for (uint32_t n = 0; n < count; ++n) {
             if (!(vflags & (1u << n))) continue;
             const NeighTerm t = neigh_term(fp, b, i, n, K);
@@ -425,21 +454,28 @@ RT_D V3 gather_pixel(const RAdjView& a, const FrameParams& fp, const Bufs& b, ui
             const V3 wn = dl * cp.f * (wa / (pp * E * D));
             pairs[static_cast<size_t>(n) * P + i] = make_float4(wn.x, wn.y, wn.z, 1.0f);
         }
-        return splat(0.0f);
+    } else {
+        item.fpv = sg.val;
+        item.pq = pp * ps;
+        item.canon_mis = canon_mis;
+        item.d = fp.k == 0 ? 0.0f : D;
+        V3 suffix_contrib = splat(0.0f);
+        for (uint32_t n = 0; n < count; ++n) {
+            const float4 c = pairs[static_cast<size_t>(n) * P + i];
+            if (c.w != 0.0f) suffix_contrib = suffix_contrib + xyz(c);
+        }
+        const V3 gather = suffix_contrib * sg.val / pp;
+        item.gather = gather / E;
     }
-    seg_prefix(a, fp, cp, sg);
-    const V3 fpv = sg.val;
-    seg_suffix(a, fp, cs, sg);
-    const V3 canon = fpv * sg.val / (pp * ps);
-    V3 suffix_contrib = splat(0.0f);
-    for (uint32_t n = 0; n < count; ++n) {
-        const float4 c = pairs[static_cast<size_t>(n) * P + i];
-        if (c.w != 0.0f) suffix_contrib = suffix_contrib + xyz(c);
-    }
-    V3 gather = suffix_contrib * fpv / pp;
-    gather = gather / E;
-    V3 result = gather + (canon * canon_mis);
-    return result / D;
+    return true;
+}
+
+RT_D void store_pixel(float* out, uint32_t i, V3 value) {
+    V3 L = splat(0.0f) + value;
+    if (nonfinite(L)) L = splat(0.0f);
+    out[3 * i] = L.x;
+    out[3 * i + 1] = L.y;
+    out[3 * i + 2] = L.z;
 }
 
 // the gradient sink of a block: all parameters in shared memory when they fit
@@ -466,27 +502,68 @@ struct BlockSink {
     }
 };
 
+// A block of two warps takes a group of 128 pixels: all of them up to the canonical
+// suffix first (neighbour weights and prefixes, about as long for each), then the
+// suffixes, whose lengths differ, a lane taking the next one when its own ends.
+// Bound by the suffixes' divergent traversal and its latency, so by the warps in
+// flight: 14 blocks, 72 registers.  8 views of 512 x 512, backward / forward ms: a
+// thread a pixel at its own registers 8.25 / 3.66, at 64 registers 6.46 / 3.26; so
+// 3.83 / 2.20, with 10 blocks 5.23 / 2.55, 20 blocks 4.27 / 2.36, 128 threads a
+// group 5.44 / 2.71, 32 threads 4.74 / 2.51, groups of 256 pixels 4.63 / 2.64.  The
+// group sets how the gradients' float sums are split, as in the path tracer's
+// adjoint, and stays at what a block of 128 threads had.
+constexpr uint32_t kGroup = 128;
+constexpr int kGroupThreads = 64;
+
 template <bool kGrad>
-__global__ void __launch_bounds__(kPassBlock) k_restir_adjoint(RAdjView a, FrameParams fp, Bufs b, const float* d_img,
-                                                               float* out, float4* pairs, float* g_mat, float* g_em,
-                                                               int use_shared) {
+__global__ void __launch_bounds__(kGroupThreads, 14) k_restir_adjoint(RAdjView a, FrameParams fp, Bufs b,
+                                                                      const float* d_img, float* out, float4* pairs,
+                                                                      float* g_mat, float* g_em, int use_shared) {
     extern __shared__ float shm[];
+    __shared__ SuffixItem<kGrad> items[kGroup];
+    __shared__ uint32_t num_items, taken;
     BlockSink bs{GradSink{kGrad && use_shared ? shm : nullptr, g_mat, g_em, a.num_mats},
                  kGrad && use_shared ? shm : nullptr, a.num_mats * kMatGrad + a.eval.num_emitters * kEmGrad};
+    if (threadIdx.x == 0) num_items = taken = 0;
     bs.begin();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    __syncthreads();
     const uint32_t P = pixel_count(fp);
-    if (i < P) {
+    const uint32_t first = blockIdx.x * kGroup, end = min(first + kGroup, P);
+    for (uint32_t i = first + threadIdx.x; i < end; i += blockDim.x) {
+        SuffixItem<kGrad> item;
+        V3 value;
+        bool suffix = false;
         if (kGrad) {
             for (uint32_t n = 0; n < fp.k; ++n) pairs[static_cast<size_t>(n) * P + i] = make_float4(0.f, 0.f, 0.f, 0.f);
             const V3 dl = V3{d_img[3 * i], d_img[3 * i + 1], d_img[3 * i + 2]};
-            if (!nonfinite(dl) && !is_zero(dl)) gather_pixel<true>(a, fp, b, i, dl, &bs.sink, pairs);
+            if (!nonfinite(dl) && !is_zero(dl)) suffix = gather_pixel(a, fp, b, i, dl, &bs.sink, pairs, value, item);
         } else {
-            V3 L = splat(0.0f) + gather_pixel<false>(a, fp, b, i, splat(0.0f), nullptr, pairs);
-            if (nonfinite(L)) L = splat(0.0f);
-            out[3 * i] = L.x;
-            out[3 * i + 1] = L.y;
-            out[3 * i + 2] = L.z;
+            suffix = gather_pixel(a, fp, b, i, splat(0.0f), static_cast<GradSink*>(nullptr), pairs, value, item);
+            if (!suffix) store_pixel(out, i, value);
+        }
+        if (suffix) items[atomicAdd(&num_items, 1u)] = item;
+    }
+    __syncthreads();
+    GroupPool pool{0, num_items, &taken};
+    SuffixPath<kGrad> path;
+    uint32_t cur = 0xffffffffu;  // the lane's item
+    while (true) {
+        const unsigned idle = __ballot_sync(0xffffffffu, cur == 0xffffffffu);
+        if (idle) {
+            const bool more = pool.more();
+            if (idle == 0xffffffffu && !more) break;
+            if (more) {
+                const uint32_t k = pool.take(cur == 0xffffffffu);
+                if (k != 0xffffffffu) {
+                    cur = k;
+                    path.begin(a, ld_suffix(b.gather_cs[items[k].pixel].sample));
+                }
+            }
+        }
+        if (cur != 0xffffffffu && !path.step(a, fp)) {
+            if constexpr (kGrad) path.sg.emit(items[cur].w, &bs.sink);
+            else store_pixel(out, items[cur].pixel, items[cur].pixel_value(path.sg.val));
+            cur = 0xffffffffu;
         }
     }
     bs.end();
@@ -495,10 +572,12 @@ __global__ void __launch_bounds__(kPassBlock) k_restir_adjoint(RAdjView a, Frame
 // one neighbour term per thread: forward, its value at theta; backward, the
 // gradient of its shifted throughput T_n (.) R_n under the weight the pixel
 // kernel wrote.  Only slots below the pixel's neighbour count (written by the
-// frame's query for every pixel) are read.
+// frame's query for every pixel) are read.  8 blocks of 128 (64 registers) instead
+// of 4: 1.60 -> 1.46 ms forward, 1.45 -> 1.34 backward (8 views of 512 x 512);
+// handing R_n's paths to lanes as they fall idle took 1.64 and 1.46.
 template <bool kGrad>
-__global__ void __launch_bounds__(kPassBlock) k_restir_pairs(RAdjView a, FrameParams fp, Bufs b, float4* pairs,
-                                                             float* g_mat, float* g_em, int use_shared) {
+__global__ void __launch_bounds__(kPassBlock, 8) k_restir_pairs(RAdjView a, FrameParams fp, Bufs b, float4* pairs,
+                                                                float* g_mat, float* g_em, int use_shared) {
     extern __shared__ float shm[];
     BlockSink bs{GradSink{kGrad && use_shared ? shm : nullptr, g_mat, g_em, a.num_mats},
                  kGrad && use_shared ? shm : nullptr, a.num_mats * kMatGrad + a.eval.num_emitters * kEmGrad};
@@ -568,7 +647,7 @@ void restir_adjoint_forward(const SceneView& eval, const crisb_material* frame_m
     if (fp.k > 0)
         k_restir_pairs<false><<<(P * fp.k + kPassBlock - 1) / kPassBlock, kPassBlock, 0, st>>>(a, fp, b, pairs, nullptr,
                                                                                               nullptr, 0);
-    k_restir_adjoint<false><<<(P + kPassBlock - 1) / kPassBlock, kPassBlock, 0, st>>>(a, fp, b, nullptr, out, pairs,
+    k_restir_adjoint<false><<<(P + kGroup - 1) / kGroup, kGroupThreads, 0, st>>>(a, fp, b, nullptr, out, pairs,
                                                                                        nullptr, nullptr, 0);
 }
 
@@ -579,9 +658,10 @@ void restir_adjoint_backward(const SceneView& eval, const crisb_material* frame_
     const RAdjView a = make_view(eval, frame_mats, frame_emitters, num_mats);
     const uint32_t P = fp.width * fp.height;
     const size_t sh_bytes = (static_cast<size_t>(num_mats) * kMatGrad + eval.num_emitters * kEmGrad) * sizeof(float);
-    const int use_shared = sh_bytes <= 48u * 1024u ? 1 : 0;
+    const int use_shared = sh_bytes <= kSharedGradBytes ? 1 : 0;
     const size_t shb = use_shared ? sh_bytes : 0;
-    k_restir_adjoint<true><<<(P + kPassBlock - 1) / kPassBlock, kPassBlock, shb, st>>>(a, fp, b, d_img, nullptr, pairs,
+    allow_shared_grads(reinterpret_cast<const void*>(k_restir_adjoint<true>), shb);
+    k_restir_adjoint<true><<<(P + kGroup - 1) / kGroup, kGroupThreads, shb, st>>>(a, fp, b, d_img, nullptr, pairs,
                                                                                        g_mat, g_em, use_shared);
     if (fp.k > 0)
         k_restir_pairs<true><<<(P * fp.k + kPassBlock - 1) / kPassBlock, kPassBlock, shb, st>>>(a, fp, b, pairs, g_mat,
