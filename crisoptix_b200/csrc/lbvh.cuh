@@ -217,14 +217,6 @@ __global__ void k_emit(Work w, int leaf_max) {
     w.nodes[i] = nd;
 }
 
-// leaf order -> primitive index from the sorted keys
-__global__ void k_order(Work w) {
-    const uint32_t n = *w.n;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    w.order[i] = static_cast<uint32_t>(w.keys[i] & 0xFFFFFFFFull);
-}
-
 #endif  // CRISB_LBVH_KERNELS
 
 }  // namespace lbvh
