@@ -19,6 +19,9 @@
 #include "records.cuh"
 
 namespace crisb {
+// search.cu: gives back what the endpoint search keeps in the current context
+void trim_search_workspace();
+
 namespace {
 
 thread_local std::string g_last_error;
@@ -71,7 +74,13 @@ struct DevBuf {
     void alloc(size_t count) {
         release();
         if (count == 0) count = 1;
-        check(cudaMalloc(&p, count * sizeof(T)), "cudaMalloc");
+        cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+        if (e == cudaErrorMemoryAllocation) {  // again without what the endpoint search keeps
+            cudaGetLastError();
+            trim_search_workspace();
+            e = cudaMalloc(&p, count * sizeof(T));
+        }
+        check(e, "cudaMalloc");
         n = count;
     }
     void upload(const T* src, size_t count) {
@@ -769,7 +778,7 @@ struct crisb_renderer {
     // Shift jobs: the list and the results have a slot for every possible
     // job (4 + 16 bytes); the machines' job records and ray queues (96 bytes
     // a job) hold jobs_per_pixel x P jobs, and a pass's jobs beyond them run
-    // in the overflow kernel -- the same results, traced in place.  A 1080p
+    // on the persistent kernel -- the same results, traced in place.  A 1080p
     // frame of the large workload runs about 2.5 jobs per pixel over all its
     // passes, against 16 slots; a capacity of 1 to 4 jobs per pixel renders
     // it within 1% of the same time.
@@ -1143,6 +1152,7 @@ int crisb_scene_create(const crisb_scene_desc* desc, crisb_scene** out) {
 
 int crisb_scene_destroy(crisb_scene* scene) {
     delete scene;
+    trim_search_workspace();
     return CRISB_OK;
 }
 

@@ -247,8 +247,16 @@ namespace {
 // between calls up to kKeepBytes.  The default pool gives its memory back whenever
 // the device is waited for, and a search then spent 0.8 of 1.25 ms (262,144 entries)
 // reserving it again.  Pool allocations are safe from any thread and on any stream;
-// memory no longer in proportion to the calls made goes back before the next.
+// memory out of proportion to a call goes back before it, all of it when a scene is
+// destroyed or the library runs out of memory (trim_search_workspace).
 constexpr uint64_t kKeepBytes = 512ull << 20;
+
+// pool management touches no stream: allowed while another thread captures one
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 
 std::mutex g_pool_mutex;
 std::vector<std::pair<unsigned long long, cudaMemPool_t>> g_pools;  // (context id, pool)
@@ -260,6 +268,7 @@ cudaMemPool_t workspace_pool() {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
     for (const auto& p : g_pools)
         if (p.first == ctx) return p.second;
+    const RelaxedCapture relaxed;
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -285,8 +294,10 @@ cudaError_t workspace_alloc(void** p, size_t bytes, cudaStream_t st) {
     if (!pool) return cudaMallocAsync(p, bytes, st);
     uint64_t held = 0;
     if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
-        held > (64ull << 20) && held / 4 > bytes)
-        cudaMemPoolTrimTo(pool, 2 * bytes);
+        held > (64ull << 20) && held / 4 > bytes) {
+        const RelaxedCapture relaxed;
+        if (cudaMemPoolTrimTo(pool, 2 * bytes) != cudaSuccess) cudaGetLastError();
+    }
     const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
     if (e == cudaSuccess) return e;
     cudaGetLastError();
@@ -294,6 +305,16 @@ cudaError_t workspace_alloc(void** p, size_t bytes, cudaStream_t st) {
 }
 
 }  // namespace
+
+namespace crisb {
+void trim_search_workspace() {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    unsigned long long ctx = 0;
+    if (g_pools.empty() || current_context_id(&ctx) != cudaSuccess) return;
+    for (const auto& p : g_pools)
+        if (p.first == ctx && p.second && cudaMemPoolTrimTo(p.second, 0) != cudaSuccess) cudaGetLastError();
+}
+}  // namespace crisb
 
 extern "C" int crisb_endpoint_search(const float* entries_dev, uint32_t n_entries, const float* queries_dev,
                                      uint32_t n_queries, uint32_t k, crisb_neighbor_rec* out_dev, uint32_t* count_dev,

@@ -448,8 +448,9 @@ int crisb_trace_rays(const crisb_scene* scene, const float* rays_dev,
  * receives the k nearest entries j with |p_j - q| <= radius_j, ordered by
  * (distance, entry index), unused slots zeroed; count_dev[q] their number.
  * k in [1, 31].  out_dev and count_dev must be 4-byte aligned.
- * Scratch comes from the stream-ordered allocator (cudaMallocAsync /
- * cudaFreeAsync on `stream`); the call is asynchronous.  A query that hits
+ * Scratch comes from a stream-ordered pool of the library (up to 512 MiB stay
+ * reserved for the next call, until a scene is destroyed; in a captured call,
+ * from the graph's own memory); the call is asynchronous.  A query that hits
  * the traversal's visit cap or stack depth keeps the neighbours found so far
  * and marks the search error word, which crisb_endpoint_search_status reads
  * (the reference's OptiX query has no such cap and reports nothing). */

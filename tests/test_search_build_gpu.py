@@ -106,3 +106,19 @@ def test_captured_search_replays(cuda_device):
         assert out.cpu().numpy().tobytes() == ref.tobytes()
         assert (cnt.cpu().numpy().view(np.uint32) == rc).all()
         gpu_search(*make_case(32, n_entries=7000, n_queries=50), 8)
+
+
+def test_kept_memory_goes_back_with_a_scene(cuda_device):
+    """The memory kept between searches is given back when a scene is destroyed."""
+    from crisoptix_b200 import Scene, scenes
+
+    e, q = case(1, 600000)
+    gpu_search(e, q, 4)
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    held = torch.cuda.mem_get_info()[0]
+    sc = Scene(scenes.cornell_box()[0])
+    del sc
+    torch.cuda.synchronize()
+    # the workspace of 600,000 entries is 100 MB and more
+    assert torch.cuda.mem_get_info()[0] >= held + (64 << 20)
