@@ -480,8 +480,8 @@ def run_crisb(args):
                  "trace_ms": passes["trace_ms"],
                  "rays_per_s": n_rays / (passes["trace_ms"] / 1000.0) if passes["trace_ms"] > 0 else None,
                  "bvh": sc.bvh_info(),
-                 "note": "closest / shadow queue traversal kernels of the path and shift machines; rays of shift "
-                         "jobs left for the last shift round are traced inside the step kernel"}
+                 "note": "closest / shadow queue traversal kernels of the path and shift machines and the persistent "
+                         "path kernels, which shade too; the persistent shift kernel's rays are in shift_ms"}
     phases = {k: passes[k] for k in ("trace_ms", "shade_ms", "shift_ms", "resample_ms", "search_ms", "other_ms")}
     pass_ms = {k[:-3]: passes[k] for k in keys[:6]}
     if dist:
