@@ -432,8 +432,9 @@ int crisb_scene_read_triangles(const crisb_scene* scene, float* positions,
 
 /* Closest-hit (any_hit == 0) or occlusion (any_hit != 0) query over the
  * scene BVH for n rays given as device arrays; ray k is
- * rays[8k..8k+7] = (ox, oy, oz, tmin, dx, dy, dz, tmax).  Hits are written
- * to the device array hits (occlusion: prim = 1 occluded, 0 free). */
+ * rays[8k..8k+7] = (ox, oy, oz, tmin, dx, dy, dz, tmax).  A direction may
+ * have any length; t counts in units of it.  Hits are written to the device
+ * array hits (occlusion: prim = 1 occluded, 0 free). */
 int crisb_trace_rays(const crisb_scene* scene, const float* rays_dev,
                      crisb_trace_hit* hits_dev, uint32_t n, int any_hit,
                      void* stream);
