@@ -178,7 +178,7 @@ struct FrozenPath {
 // The pixels' paths of a pool: a lane takes the next pixel when its path ends and
 // traces one ray of either kind a turn.  kGrad: `d_img` is the image's adjoint,
 // whose zero and non-finite pixels trace nothing; else `out` is the image.
-template <bool kGrad, class Pool>
+template <bool kGrad, int kFmt, class Pool>
 RT_D void frozen_pixels(const AdjView& a, const FrameParams& fp, Pool pool, const float* d_img, float* out,
                         GradSink* sink) {
     FrozenPath<kGrad> path;
@@ -206,7 +206,7 @@ RT_D void frozen_pixels(const AdjView& a, const FrameParams& fp, Pool pool, cons
             }
         }
         if (pixel != 0xffffffffu) {
-            const TraceResult h = traverse_ray(a.eval, path.o, path.d, 1e-3f, path.tmax, path.shadow);
+            const TraceResult h = traverse_ray<kFmt>(a.eval, path.o, path.d, 1e-3f, path.tmax, path.shadow);
             if (!path.step(a, fp, h, dl, tl, sink)) {
                 if (!kGrad) {
                     V3 L = path.radiance;
@@ -222,8 +222,9 @@ RT_D void frozen_pixels(const AdjView& a, const FrameParams& fp, Pool pool, cons
 }
 
 // 6 resident blocks per SM (80 registers; 4 and 5 blocks: 2-4% slower)
+template <int kFmt>
 __global__ void __launch_bounds__(kPassBlock, 6) k_frozen_forward(AdjView a, FrameParams fp, float* out) {
-    frozen_pixels<false>(a, fp, PixelPool(fp.width * fp.height), nullptr, out, nullptr);
+    frozen_pixels<false, kFmt>(a, fp, PixelPool(fp.width * fp.height), nullptr, out, nullptr);
 }
 
 // Backward: a block of two warps per group of 128 pixels, whose lanes take the
@@ -238,6 +239,7 @@ __global__ void __launch_bounds__(kPassBlock, 6) k_frozen_forward(AdjView a, Fra
 constexpr uint32_t kGroup = 128;
 constexpr int kGroupThreads = 64;
 
+template <int kFmt>
 __global__ void __launch_bounds__(kGroupThreads, 10) k_frozen_backward(AdjView a, FrameParams fp, const float* d_img,
                                                                       float* g_mat, float* g_em, int use_shared) {
     extern __shared__ float sh[];
@@ -249,7 +251,7 @@ __global__ void __launch_bounds__(kGroupThreads, 10) k_frozen_backward(AdjView a
     __syncthreads();
     GradSink sink{use_shared ? sh : nullptr, g_mat, g_em, a.num_mats};
     const uint32_t first = blockIdx.x * kGroup;
-    frozen_pixels<true>(a, fp, GroupPool{first, min(kGroup, fp.width * fp.height - first), &taken}, d_img, nullptr, &sink);
+    frozen_pixels<true, kFmt>(a, fp, GroupPool{first, min(kGroup, fp.width * fp.height - first), &taken}, d_img, nullptr, &sink);
     if (use_shared) {
         __syncthreads();
         for (uint32_t k = threadIdx.x; k < n_sh; k += blockDim.x) {
@@ -272,26 +274,40 @@ unsigned resident_blocks(const void* kernel) {
     return 148u * 4u;
 }
 
-}  // namespace
-
-// host side, called from api.cu
-void adjoint_forward(const SceneView& eval, const crisb_material* sample_mats, uint32_t num_mats,
-                     const FrameParams& fp, float* out, cudaStream_t st) {
+template <int kFmt>
+void forward(const SceneView& eval, const crisb_material* sample_mats, uint32_t num_mats, const FrameParams& fp,
+             float* out, cudaStream_t st) {
     const AdjView a{eval, sample_mats, num_mats, eval.num_emitters};
     const uint32_t P = fp.width * fp.height;
-    static const unsigned resident = resident_blocks(reinterpret_cast<const void*>(k_frozen_forward));
-    k_frozen_forward<<<std::min((P + kPassBlock - 1) / kPassBlock, resident), kPassBlock, 0, st>>>(a, fp, out);
+    static const unsigned resident = resident_blocks(reinterpret_cast<const void*>(k_frozen_forward<kFmt>));
+    k_frozen_forward<kFmt><<<std::min((P + kPassBlock - 1) / kPassBlock, resident), kPassBlock, 0, st>>>(a, fp, out);
 }
 
-void adjoint_backward(const SceneView& eval, const crisb_material* sample_mats, uint32_t num_mats,
-                      const FrameParams& fp, const float* d_img, float* g_mat, float* g_em, cudaStream_t st) {
+template <int kFmt>
+void backward(const SceneView& eval, const crisb_material* sample_mats, uint32_t num_mats, const FrameParams& fp,
+              const float* d_img, float* g_mat, float* g_em, cudaStream_t st) {
     const AdjView a{eval, sample_mats, num_mats, eval.num_emitters};
     const uint32_t P = fp.width * fp.height;
     const size_t sh_bytes = (static_cast<size_t>(num_mats) * kMatGrad + eval.num_emitters * kEmGrad) * sizeof(float);
     const int use_shared = sh_bytes <= kSharedGradBytes ? 1 : 0;
     const size_t shb = use_shared ? sh_bytes : 0;
-    allow_shared_grads(reinterpret_cast<const void*>(k_frozen_backward), shb);
-    k_frozen_backward<<<(P + kGroup - 1) / kGroup, kGroupThreads, shb, st>>>(a, fp, d_img, g_mat, g_em, use_shared);
+    allow_shared_grads(reinterpret_cast<const void*>(k_frozen_backward<kFmt>), shb);
+    k_frozen_backward<kFmt><<<(P + kGroup - 1) / kGroup, kGroupThreads, shb, st>>>(a, fp, d_img, g_mat, g_em, use_shared);
+}
+
+}  // namespace
+
+// host side, called from api.cu
+void adjoint_forward(const SceneView& eval, const crisb_material* sample_mats, uint32_t num_mats,
+                     const FrameParams& fp, float* out, cudaStream_t st) {
+    const auto run = eval.qnodes ? forward<kFmtAny> : forward<kFmtWide4>;
+    run(eval, sample_mats, num_mats, fp, out, st);
+}
+
+void adjoint_backward(const SceneView& eval, const crisb_material* sample_mats, uint32_t num_mats,
+                      const FrameParams& fp, const float* d_img, float* g_mat, float* g_em, cudaStream_t st) {
+    const auto run = eval.qnodes ? backward<kFmtAny> : backward<kFmtWide4>;
+    run(eval, sample_mats, num_mats, fp, d_img, g_mat, g_em, st);
 }
 
 }  // namespace crisb

@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kPassBlock, 8) k_shift_step(SceneView s, Frame
 // The jobs on persistent warps, as the path flows (wavefront.cu): the whole list
 // (round < 0), or the jobs whose rays round `round` traced and the list's entries
 // beyond the machines' records.
-template <bool kTex>
+template <bool kTex, int kFmt>
 __global__ void __launch_bounds__(kPassBlock, 5) k_shift(SceneView s, FrameParams fp, Bufs b, int mode, int round) {
     constexpr unsigned kFull = 0xffffffffu;
     const uint32_t all = *b.job_count;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kPassBlock, 5) k_shift(SceneView s, FrameParam
         if (!traced && job.phase > kJobStart) {
             const bool shadow = job.phase == kJobShadow;
             count_ray_kind(s, shadow);
-            h = traverse_ray(s, job.o, job.d, 1e-3f, shadow ? job.tmax : 1e16f, shadow);
+            h = traverse_ray<kFmt>(s, job.o, job.d, 1e-3f, shadow ? job.tmax : 1e16f, shadow);
             traced = true;
         }
     }
@@ -1013,7 +1013,7 @@ RT_D void prefix_tail(const FrameParams& fp, const Bufs& b, float* out, uint32_t
 // scene against a thread a pixel (2.0 G rays/s).  4 / 5 / 6 / 7 resident blocks
 // (115, 94, 80, 72 registers): 1.25 / 1.15 / 1.13 / 1.19 ms; refilling only once 8 or
 // 16 lanes are idle: 1.15 / 1.23 ms.
-template <bool kTex>
+template <bool kTex, int kFmt>
 __global__ void __launch_bounds__(kPassBlock, 5) k_path_tracer(SceneView s, FrameParams fp, float* out) {
     PixelPool pool(pixel_count(fp));
     CompletePath path;
@@ -1035,7 +1035,7 @@ __global__ void __launch_bounds__(kPassBlock, 5) k_path_tracer(SceneView s, Fram
         }
         if (pixel != 0xffffffffu) {
             count_ray_kind(s, path.shadow);
-            const TraceResult h = traverse_ray(s, path.o, path.d, 1e-3f, path.tmax, path.shadow);
+            const TraceResult h = traverse_ray<kFmt>(s, path.o, path.d, 1e-3f, path.tmax, path.shadow);
             if (!path.template step<kTex>(s, fp, h)) {
                 V3 L = path.radiance;
                 if (nonfinite(L)) L = splat(0.0f);
@@ -1160,24 +1160,24 @@ __global__ void __launch_bounds__(kPassBlock, kResampleMinBlocks) k_prefix_combi
     prefix_tail(fp, b, out, i, cur, true);
 }
 
-template <bool kTex>
-unsigned path_tracer_grid() {
-    static const unsigned g = persistent_grid(reinterpret_cast<const void*>(k_path_tracer<kTex>));
-    return g;
+template <bool kTex, int kFmt>
+void launch_path_tracer(const SceneView& s, const FrameParams& fp, float* out, cudaStream_t st) {
+    static const unsigned g = persistent_grid(reinterpret_cast<const void*>(k_path_tracer<kTex, kFmt>));
+    k_path_tracer<kTex, kFmt><<<std::min(g, grid_for(fp.width * fp.height)), kPassBlock, 0, st>>>(s, fp, out);
 }
 
 struct ShiftGrids {
     unsigned begin, step, persistent;
 };
 
-template <bool kTex>
+template <bool kTex, int kFmt>
 const ShiftGrids& shift_grids() {
     static std::once_flag once;
     static ShiftGrids g{};
     std::call_once(once, [] {
         g.begin = persistent_grid(reinterpret_cast<const void*>(k_shift_begin<kTex>));
         g.step = persistent_grid(reinterpret_cast<const void*>(k_shift_step<kTex>));
-        g.persistent = persistent_grid(reinterpret_cast<const void*>(k_shift<kTex>));
+        g.persistent = persistent_grid(reinterpret_cast<const void*>(k_shift<kTex, kFmt>));
     });
     return g;
 }
@@ -1213,10 +1213,10 @@ void take_counters(Bufs& b, Counters& c) {
 }
 
 // the shift jobs of the list: rounds of trace / step, then persistent warps
-template <bool kTex>
+template <bool kTex, int kFmt>
 void run_shift_jobs_as(const SceneView& s, const FrameParams& fp, const Bufs& b, int mode, cudaStream_t st,
                        Marker* m) {
-    const ShiftGrids& g = shift_grids<kTex>();
+    const ShiftGrids& g = shift_grids<kTex, kFmt>();
     const int rounds = shift_rounds(fp);
     if (rounds > 0) {
         k_shift_begin<kTex><<<g.begin, kPassBlock, 0, st>>>(s, fp, b, mode);
@@ -1232,7 +1232,7 @@ void run_shift_jobs_as(const SceneView& s, const FrameParams& fp, const Bufs& b,
             MARK(kClsShift);
         }
     }
-    k_shift<kTex><<<g.persistent, kPassBlock, 0, st>>>(s, fp, b, mode, rounds - 1);
+    k_shift<kTex, kFmt><<<g.persistent, kPassBlock, 0, st>>>(s, fp, b, mode, rounds - 1);
     MARK(kClsShift);
 }
 
@@ -1241,10 +1241,10 @@ void run_shift_jobs_as(const SceneView& s, const FrameParams& fp, const Bufs& b,
 // 5 resident blocks per SM)
 void run_shift_jobs(const SceneView& s0, const FrameParams& fp, const Bufs& b, int mode, cudaStream_t st, Marker* m) {
     const SceneView s = shift_view(s0);
-    if (s.mat_tex)
-        run_shift_jobs_as<true>(s, fp, b, mode, st, m);
-    else
-        run_shift_jobs_as<false>(s, fp, b, mode, st, m);
+    const auto run = s.qnodes ? (s.mat_tex ? run_shift_jobs_as<true, kFmtAny>
+                                           : run_shift_jobs_as<false, kFmtAny>)
+                              : (s.mat_tex ? run_shift_jobs_as<true, kFmtWide4> : run_shift_jobs_as<false, kFmtWide4>);
+    run(s, fp, b, mode, st, m);
 }
 
 }  // namespace
@@ -1254,9 +1254,11 @@ uint32_t shift_launches(const FrameParams& fp) { return 1 + 2 * static_cast<uint
 void launch_prefix_gen_temp_split(const SceneView& s, const FrameParams& fp, Bufs b, Counters& c, float* out,
                                   cudaStream_t st, Marker* m) {
     if (fp.p.renderer_type == CRISB_RENDERER_PATH_TRACER) {
-        const unsigned most = grid_for(fp.width * fp.height);
-        if (s.mat_tex) k_path_tracer<true><<<std::min(path_tracer_grid<true>(), most), kPassBlock, 0, st>>>(s, fp, out);
-        else k_path_tracer<false><<<std::min(path_tracer_grid<false>(), most), kPassBlock, 0, st>>>(s, fp, out);
+        const auto launch = s.qnodes ? (s.mat_tex ? launch_path_tracer<true, kFmtAny>
+                                                  : launch_path_tracer<false, kFmtAny>)
+                                     : (s.mat_tex ? launch_path_tracer<true, kFmtWide4>
+                                                  : launch_path_tracer<false, kFmtWide4>);
+        launch(s, fp, out, st);
         MARK(kClsOther);
         return;
     }

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kPassBlock, 5) k_flow_shade(SceneView s, Frame
 // side in one traversal), steps, and takes another path when it has ended:
 // every pixel's path from its start (round < 0), or the paths whose rays are
 // queued for round `round`.
-template <int kFlow, bool kTex>
+template <int kFlow, bool kTex, int kFmt>
 __global__ void __launch_bounds__(kPassBlock, 5) k_flow(SceneView s, FrameParams fp, Bufs b, int round) {
     constexpr unsigned kFull = 0xffffffffu;
     const bool fresh = round < 0;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kPassBlock, 5) k_flow(SceneView s, FrameParams
         if (path.phase > kPhStart) {
             const bool shadow = path.phase == kPhShadow;
             count_ray_kind(s, shadow);
-            h = traverse_ray(s, path.o, path.d, 1e-3f, shadow ? path.tmax : 1e16f, shadow);
+            h = traverse_ray<kFmt>(s, path.o, path.d, 1e-3f, shadow ? path.tmax : 1e16f, shadow);
             traced = true;
         }
     }
@@ -140,9 +140,9 @@ int most_rays(const crisb_params& p, int flow) {
 // the parameters say: temporal reuse keeps prefixes of other lengths)
 bool needs_tail(const crisb_params& p, int flow, int rounds) { return flow == 1 || rounds < most_rays(p, flow); }
 
-template <int kFlow, bool kTex>
+template <int kFlow, bool kTex, int kFmt>
 void launch_flow_as(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m) {
-    static const unsigned g_flow = persistent_grid(reinterpret_cast<const void*>(k_flow<kFlow, kTex>));
+    static const unsigned g_flow = persistent_grid(reinterpret_cast<const void*>(k_flow<kFlow, kTex, kFmt>));
     static const unsigned g_shade = persistent_grid(reinterpret_cast<const void*>(k_flow_shade<kFlow, kTex>));
     const unsigned most = grid_for(fp.width * fp.height);  // a path a pixel
     const int rounds = flow_rounds(fp, kFlow, kTex);
@@ -159,14 +159,17 @@ void launch_flow_as(const SceneView& s, const FrameParams& fp, const Bufs& b, cu
         if (m) m->mark(kClsShade, st);
     }
     if (rounds > 0 && !needs_tail(fp.p, kFlow, rounds)) return;
-    k_flow<kFlow, kTex><<<std::min(g_flow, most), kPassBlock, 0, st>>>(s, fp, b, rounds > 0 ? rounds : -1);
+    k_flow<kFlow, kTex, kFmt><<<std::min(g_flow, most), kPassBlock, 0, st>>>(s, fp, b, rounds > 0 ? rounds : -1);
     if (m) m->mark(kClsTrace, st);
 }
 
 template <int kFlow>
 void launch_flow(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaStream_t st, Marker* m) {
-    if (s.mat_tex) launch_flow_as<kFlow, true>(s, fp, b, st, m);
-    else launch_flow_as<kFlow, false>(s, fp, b, st, m);
+    const auto launch = s.qnodes ? (s.mat_tex ? launch_flow_as<kFlow, true, kFmtAny>
+                                              : launch_flow_as<kFlow, false, kFmtAny>)
+                                 : (s.mat_tex ? launch_flow_as<kFlow, true, kFmtWide4>
+                                              : launch_flow_as<kFlow, false, kFmtWide4>);
+    launch(s, fp, b, st, m);
 }
 
 }  // namespace
