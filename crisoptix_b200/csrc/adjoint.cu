@@ -227,21 +227,24 @@ __global__ void __launch_bounds__(kPassBlock, 6) k_frozen_forward(AdjView a, Fra
     frozen_pixels<false, kFmt>(a, fp, PixelPool(fp.width * fp.height), nullptr, out, nullptr);
 }
 
-// Backward: a block of two warps per group of 128 pixels, whose lanes take the
-// group's pixels in turn and whose gradients gather in one shared-memory block of
-// all parameters (12 KB for the large scene) that reaches global memory once.
-// The group, not the block, sets how the gradients' float sums are split:
-// larger ones, as persistent warps would have, change them by 2e-5 through what a
-// global sum of 1e9 takes from each addition.  Forward and backward of 8 views of
-// 512 x 512: 11.3 ms with 64 threads a group (10 blocks per SM, 96 registers), 12.3
-// with 128, 11.9 with 96, 11.7 with 32; 15.9 with a thread a pixel, each warp
-// running until its longest path ended.
+// Backward: a block per group of 128 pixels, whose lanes take the group's pixels in
+// turn and whose gradients gather in one shared-memory block of all parameters (12 KB
+// for the large scene) that reaches global memory once.  The group, not the block,
+// sets how the gradients' float sums are split: larger ones, as persistent warps
+// would have, change them by 2e-5 through what a global sum of 1e9 takes from each
+// addition.  Forward and backward of 8 views of 512 x 512: 11.3 ms with 64 threads a
+// group (10 blocks per SM, 96 registers), 12.3 with 128, 11.9 with 96, 11.7 with 32;
+// 15.9 with a thread a pixel, each warp running until its longest path ended.
+// Images whose groups are all resident at once with a thread a pixel take that
+// instead: two pixels a lane then only make the chain longer (one view, backward,
+// 64 x 64 283 against 431 us, 256 x 256 413 / 509, 320 x 320, just above the line,
+// 586 / 604, 384 x 384 779 / 719).
 constexpr uint32_t kGroup = 128;
 constexpr int kGroupThreads = 64;
 
 template <int kFmt>
-__global__ void __launch_bounds__(kGroupThreads, 10) k_frozen_backward(AdjView a, FrameParams fp, const float* d_img,
-                                                                      float* g_mat, float* g_em, int use_shared) {
+__global__ void __launch_bounds__(kGroup, 5) k_frozen_backward(AdjView a, FrameParams fp, const float* d_img,
+                                                               float* g_mat, float* g_em, int use_shared) {
     extern __shared__ float sh[];
     __shared__ uint32_t taken;
     const uint32_t n_sh = a.num_mats * kMatGrad + a.num_emitters * kEmGrad;
@@ -292,7 +295,10 @@ void backward(const SceneView& eval, const crisb_material* sample_mats, uint32_t
     const int use_shared = sh_bytes <= kSharedGradBytes ? 1 : 0;
     const size_t shb = use_shared ? sh_bytes : 0;
     allow_shared_grads(reinterpret_cast<const void*>(k_frozen_backward<kFmt>), shb);
-    k_frozen_backward<kFmt><<<(P + kGroup - 1) / kGroup, kGroupThreads, shb, st>>>(a, fp, d_img, g_mat, g_em, use_shared);
+    static const unsigned resident = resident_blocks(reinterpret_cast<const void*>(k_frozen_backward<kFmt>));
+    const unsigned groups = (P + kGroup - 1) / kGroup;
+    const unsigned threads = groups <= resident ? kGroup : kGroupThreads;
+    k_frozen_backward<kFmt><<<groups, threads, shb, st>>>(a, fp, d_img, g_mat, g_em, use_shared);
 }
 
 }  // namespace
