@@ -36,6 +36,7 @@
 // factor's derivatives with dLoss/dL times the other factors (chain rule at
 // theta0) and adds them through the warp-aggregated gradient sink.
 #include "adjoint_common.cuh"
+#include "queues.cuh"
 #include "records.cuh"
 
 namespace crisb {
@@ -478,6 +479,13 @@ RT_D void store_pixel(float* out, uint32_t i, V3 value) {
     out[3 * i + 2] = L.z;
 }
 
+// a finished suffix: its gradient into the sink, or its pixel's value
+template <bool kGrad>
+RT_D void finish_suffix(const SuffixPath<kGrad>& path, const SuffixItem<kGrad>& item, GradSink* sink, float* out) {
+    if constexpr (kGrad) path.sg.emit(item.w, sink);
+    else store_pixel(out, item.pixel, item.pixel_value(path.sg.val));
+}
+
 // the gradient sink of a block: all parameters in shared memory when they fit
 struct BlockSink {
     GradSink sink;
@@ -512,15 +520,21 @@ struct BlockSink {
 // group 5.44 / 2.71, 32 threads 4.74 / 2.51, groups of 256 pixels 4.63 / 2.64.  The
 // group sets how the gradients' float sums are split, as in the path tracer's
 // adjoint, and stays at what a block of 128 threads had.
+// Images whose groups are all resident at once with a thread a pixel (kPool false: at
+// most 592 of 128 threads at up to 128 registers) have no other work to fill the idle
+// lanes with, and the wait between the two parts only adds to the chain: there each
+// lane goes on with its own suffix.  Backward / forward us of one view of the box at
+// 64 x 64: 80 / 52 instead of 121 / 72, of the room at 256 x 256 262 / 190 instead of
+// 342 / 224, at 320 x 320, above the line, 438 / 275 instead of 413 / 267.
 constexpr uint32_t kGroup = 128;
 constexpr int kGroupThreads = 64;
 
-template <bool kGrad>
-__global__ void __launch_bounds__(kGroupThreads, 14) k_restir_adjoint(RAdjView a, FrameParams fp, Bufs b,
-                                                                      const float* d_img, float* out, float4* pairs,
-                                                                      float* g_mat, float* g_em, int use_shared) {
+template <bool kGrad, bool kPool>
+__global__ void __launch_bounds__(kPool ? kGroupThreads : kGroup, kPool ? 14 : 4)
+    k_restir_adjoint(RAdjView a, FrameParams fp, Bufs b, const float* d_img, float* out, float4* pairs, float* g_mat,
+                     float* g_em, int use_shared) {
     extern __shared__ float shm[];
-    __shared__ SuffixItem<kGrad> items[kGroup];
+    __shared__ SuffixItem<kGrad> items[kPool ? kGroup : 1];
     __shared__ uint32_t num_items, taken;
     BlockSink bs{GradSink{kGrad && use_shared ? shm : nullptr, g_mat, g_em, a.num_mats},
                  kGrad && use_shared ? shm : nullptr, a.num_mats * kMatGrad + a.eval.num_emitters * kEmGrad};
@@ -541,29 +555,39 @@ __global__ void __launch_bounds__(kGroupThreads, 14) k_restir_adjoint(RAdjView a
             suffix = gather_pixel(a, fp, b, i, splat(0.0f), static_cast<GradSink*>(nullptr), pairs, value, item);
             if (!suffix) store_pixel(out, i, value);
         }
-        if (suffix) items[atomicAdd(&num_items, 1u)] = item;
+        if (!suffix) continue;
+        if constexpr (kPool) {
+            items[atomicAdd(&num_items, 1u)] = item;
+        } else {
+            SuffixPath<kGrad> path;
+            path.begin(a, ld_suffix(b.gather_cs[i].sample));
+            while (path.step(a, fp)) {
+            }
+            finish_suffix(path, item, &bs.sink, out);
+        }
     }
-    __syncthreads();
-    GroupPool pool{0, num_items, &taken};
-    SuffixPath<kGrad> path;
-    uint32_t cur = 0xffffffffu;  // the lane's item
-    while (true) {
-        const unsigned idle = __ballot_sync(0xffffffffu, cur == 0xffffffffu);
-        if (idle) {
-            const bool more = pool.more();
-            if (idle == 0xffffffffu && !more) break;
-            if (more) {
-                const uint32_t k = pool.take(cur == 0xffffffffu);
-                if (k != 0xffffffffu) {
-                    cur = k;
-                    path.begin(a, ld_suffix(b.gather_cs[items[k].pixel].sample));
+    if constexpr (kPool) {
+        __syncthreads();
+        GroupPool pool{0, num_items, &taken};
+        SuffixPath<kGrad> path;
+        uint32_t cur = 0xffffffffu;  // the lane's item
+        while (true) {
+            const unsigned idle = __ballot_sync(0xffffffffu, cur == 0xffffffffu);
+            if (idle) {
+                const bool more = pool.more();
+                if (idle == 0xffffffffu && !more) break;
+                if (more) {
+                    const uint32_t k = pool.take(cur == 0xffffffffu);
+                    if (k != 0xffffffffu) {
+                        cur = k;
+                        path.begin(a, ld_suffix(b.gather_cs[items[k].pixel].sample));
+                    }
                 }
             }
-        }
-        if (cur != 0xffffffffu && !path.step(a, fp)) {
-            if constexpr (kGrad) path.sg.emit(items[cur].w, &bs.sink);
-            else store_pixel(out, items[cur].pixel, items[cur].pixel_value(path.sg.val));
-            cur = 0xffffffffu;
+            if (cur != 0xffffffffu && !path.step(a, fp)) {
+                finish_suffix(path, items[cur], &bs.sink, out);
+                cur = 0xffffffffu;
+            }
         }
     }
     bs.end();
@@ -626,6 +650,20 @@ __global__ void __launch_bounds__(kPassBlock, 8) k_restir_pairs(RAdjView a, Fram
     bs.end();
 }
 
+// the instance for P pixels and its launch shape
+struct Launch {
+    void (*kernel)(RAdjView, FrameParams, Bufs, const float*, float*, float4*, float*, float*, int);
+    unsigned groups, threads;
+};
+
+template <bool kGrad>
+Launch launch_of(uint32_t P) {
+    static const unsigned resident = persistent_grid(reinterpret_cast<const void*>(k_restir_adjoint<kGrad, false>));
+    const unsigned groups = (P + kGroup - 1) / kGroup;
+    if (groups <= resident) return Launch{k_restir_adjoint<kGrad, false>, groups, kGroup};
+    return Launch{k_restir_adjoint<kGrad, true>, groups, kGroupThreads};
+}
+
 RAdjView make_view(const SceneView& eval, const crisb_material* frame_mats, const crisb_emitter* frame_emitters,
                    uint32_t num_mats) {
     RAdjView a;
@@ -647,8 +685,8 @@ void restir_adjoint_forward(const SceneView& eval, const crisb_material* frame_m
     if (fp.k > 0)
         k_restir_pairs<false><<<(P * fp.k + kPassBlock - 1) / kPassBlock, kPassBlock, 0, st>>>(a, fp, b, pairs, nullptr,
                                                                                               nullptr, 0);
-    k_restir_adjoint<false><<<(P + kGroup - 1) / kGroup, kGroupThreads, 0, st>>>(a, fp, b, nullptr, out, pairs,
-                                                                                       nullptr, nullptr, 0);
+    const Launch l = launch_of<false>(P);
+    l.kernel<<<l.groups, l.threads, 0, st>>>(a, fp, b, nullptr, out, pairs, nullptr, nullptr, 0);
 }
 
 void restir_adjoint_backward(const SceneView& eval, const crisb_material* frame_mats,
@@ -660,9 +698,9 @@ void restir_adjoint_backward(const SceneView& eval, const crisb_material* frame_
     const size_t sh_bytes = (static_cast<size_t>(num_mats) * kMatGrad + eval.num_emitters * kEmGrad) * sizeof(float);
     const int use_shared = sh_bytes <= kSharedGradBytes ? 1 : 0;
     const size_t shb = use_shared ? sh_bytes : 0;
-    allow_shared_grads(reinterpret_cast<const void*>(k_restir_adjoint<true>), shb);
-    k_restir_adjoint<true><<<(P + kGroup - 1) / kGroup, kGroupThreads, shb, st>>>(a, fp, b, d_img, nullptr, pairs,
-                                                                                       g_mat, g_em, use_shared);
+    const Launch l = launch_of<true>(P);
+    allow_shared_grads(reinterpret_cast<const void*>(l.kernel), shb);
+    l.kernel<<<l.groups, l.threads, shb, st>>>(a, fp, b, d_img, nullptr, pairs, g_mat, g_em, use_shared);
     if (fp.k > 0)
         k_restir_pairs<true><<<(P * fp.k + kPassBlock - 1) / kPassBlock, kPassBlock, shb, st>>>(a, fp, b, pairs, g_mat,
                                                                                                g_em, use_shared);

@@ -9,8 +9,8 @@ import numpy as np
 import pytest
 import torch
 
-from crisoptix_b200 import Scene, adjoint, default_params
-from helpers import small_sphere_room
+from crisoptix_b200 import Scene, _abi, adjoint, default_params
+from helpers import large_config_params, scene_size_of, small_sphere_room
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +55,21 @@ def test_path_tracer_adjoint(cuda_device, w, h):
         if (img > 0).all(dim=-1).any():
             break
     check_pixels(sc, desc, img, lambda d: adj.gradient([cam], d))
+
+
+# the sizes above, and those around the resampled adjoint's own line (592 groups)
+@pytest.mark.parametrize("w,h", SIZES[:-3] + [(296, 256), (296, 257), (641, 479)])
+@pytest.mark.parametrize("k", [0, 8])
+def test_resampled_adjoint(cuda_device, w, h, k):
+    desc, cam = small_sphere_room()
+    sc = Scene(desc)
+    for seed in range(64):
+        p = large_config_params(scene_size_of(desc), max_path_len=6, enable_accum=0, gather_n=1, gather_m=k + 1,
+                                gather_radius=0.3, storage=_abi.STORAGE_FP32, seed=seed)
+        adj = adjoint.RestirAdjoint(sc, w, h, p, 1)
+        frame = adj.prepare([cam], frames=3)
+        img = adj.render()
+        if (img > 0).all(dim=-1).any():
+            break
+    np.testing.assert_array_equal(img.cpu().numpy(), frame.cpu().numpy())
+    check_pixels(sc, desc, img, adj.gradient)
