@@ -152,9 +152,13 @@ RT_D float4 ld_image(const float4* p) {
     return v;
 }
 
-// Pixels [0, 4 * quads) four per thread with vector accesses (rgb 16-byte and
-// out 4-byte aligned), pixels [4 * quads, n) one per thread, a thread's next
-// pixels loaded before its present ones are stored.  What bounds it: launch and
+// kVec: pixels [0, 4 * quads) four per thread with vector accesses (rgb 16-byte and
+// out 4-byte aligned), a thread's next pixels loaded before its present ones are
+// stored, and the last few one per thread.  Else pixels one by one, kTurns of a
+// thread's loaded before they are stored, in a kernel of its own: the registers of the
+// vector loop would leave it 3 instead of 4 blocks of 512 threads per SM, and with
+// that and a pixel at a time 33.2 million unaligned pixels took 151 us, now 95.  What
+// bounds it: launch and
 // table load for small images, memory for large ones (3840x3840: 221 MB in 36 us,
 // 6.1 TB/s).  Launched beside the end of the work before it (launch_tonemap_srgb8), a
 // block copies the table, which never changes, before it waits for that work; the
@@ -164,46 +168,66 @@ RT_D float4 ld_image(const float4* p) {
 // through the read-only path (no __restrict__) or may move above the wait.
 // Back to back, before and after: 1920x1080 12.4 -> 9.4 us (the host's launch rate;
 // 12.1 without the early launch), 3840x2160 28.7 -> 22.1, 3840x3840 45.1 -> 36.2.
+template <bool kVec>
 __global__ void __launch_bounds__(kToneBlock) k_tonemap_srgb8(const float* rgb, uint8_t* out, uint32_t n,
                                                              uint32_t quads, const uint32_t* table,
                                                              uint32_t max_bits) {
     __shared__ uint32_t t[kBuckets + 1];
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    const float4* in4 = reinterpret_cast<const float4*>(rgb);
-    uint32_t* out4 = reinterpret_cast<uint32_t*>(out);
     asm volatile("griddepcontrol.launch_dependents;");
     for (uint32_t i = threadIdx.x; i <= kBuckets; i += blockDim.x) t[i] = __ldg(table + i);
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    uint64_t q = tid;
-    float4 a, b, c;
-    if (q < quads) {
-        a = ld_image(in4 + 3 * q);
-        b = ld_image(in4 + 3 * q + 1);
-        c = ld_image(in4 + 3 * q + 2);
-    }
-    __syncthreads();
-    while (q < quads) {
-        const uint64_t next = q + stride;
-        float4 na, nb, nc;
-        if (next < quads) {
-            na = ld_image(in4 + 3 * next);
-            nb = ld_image(in4 + 3 * next + 1);
-            nc = ld_image(in4 + 3 * next + 2);
+    if (kVec) {
+        const float4* in4 = reinterpret_cast<const float4*>(rgb);
+        uint32_t* out4 = reinterpret_cast<uint32_t*>(out);
+        uint64_t q = tid;
+        float4 a, b, c;
+        if (q < quads) {
+            a = ld_image(in4 + 3 * q);
+            b = ld_image(in4 + 3 * q + 1);
+            c = ld_image(in4 + 3 * q + 2);
         }
-        __stcs(out4 + 3 * q, srgb8_word(t, a, max_bits));
-        __stcs(out4 + 3 * q + 1, srgb8_word(t, b, max_bits));
-        __stcs(out4 + 3 * q + 2, srgb8_word(t, c, max_bits));
-        a = na;
-        b = nb;
-        c = nc;
-        q = next;
-    }
-    for (uint64_t i = 4 * static_cast<uint64_t>(quads) + tid; i < n; i += stride) {
-        const uint64_t o = 3 * i;
-        out[o] = static_cast<uint8_t>(srgb8_lookup(t, rgb[o], max_bits));
-        out[o + 1] = static_cast<uint8_t>(srgb8_lookup(t, rgb[o + 1], max_bits));
-        out[o + 2] = static_cast<uint8_t>(srgb8_lookup(t, rgb[o + 2], max_bits));
+        __syncthreads();
+        while (q < quads) {
+            const uint64_t next = q + stride;
+            float4 na, nb, nc;
+            if (next < quads) {
+                na = ld_image(in4 + 3 * next);
+                nb = ld_image(in4 + 3 * next + 1);
+                nc = ld_image(in4 + 3 * next + 2);
+            }
+            __stcs(out4 + 3 * q, srgb8_word(t, a, max_bits));
+            __stcs(out4 + 3 * q + 1, srgb8_word(t, b, max_bits));
+            __stcs(out4 + 3 * q + 2, srgb8_word(t, c, max_bits));
+            a = na;
+            b = nb;
+            c = nc;
+            q = next;
+        }
+        const uint64_t i = 4 * static_cast<uint64_t>(quads) + tid;
+        if (i < n)
+            for (int ch = 0; ch < 3; ++ch)
+                out[3 * i + ch] = static_cast<uint8_t>(srgb8_lookup(t, rgb[3 * i + ch], max_bits));
+    } else {
+        constexpr uint64_t kTurns = 4;
+        __syncthreads();
+        for (uint64_t i = tid; i < n; i += kTurns * stride) {
+            float v[kTurns][3];
+#pragma unroll
+            for (uint64_t k = 0; k < kTurns; ++k) {
+                const uint64_t p = i + k * stride;
+                if (p < n)
+                    for (int ch = 0; ch < 3; ++ch) v[k][ch] = rgb[3 * p + ch];
+            }
+#pragma unroll
+            for (uint64_t k = 0; k < kTurns; ++k) {
+                const uint64_t p = i + k * stride;
+                if (p < n)
+                    for (int ch = 0; ch < 3; ++ch)
+                        out[3 * p + ch] = static_cast<uint8_t>(srgb8_lookup(t, v[k][ch], max_bits));
+            }
+        }
     }
 }
 
@@ -247,11 +271,12 @@ const uint32_t* device_table() {
 }
 
 // blocks of the kernel resident on the whole device at once
+template <bool kVec>
 unsigned tone_grid_cap() {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tonemap_srgb8, kToneBlock, 0) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tonemap_srgb8<kVec>, kToneBlock, 0) == cudaSuccess &&
         sms > 0 && per_sm > 0)
         return static_cast<unsigned>(sms * per_sm);
     return 148u * 8u;
@@ -270,7 +295,8 @@ cudaError_t launch_tonemap_srgb8(const float* rgb, uint8_t* out, uint32_t n, cud
     const bool vec = (reinterpret_cast<uintptr_t>(rgb) % 16 == 0) && (reinterpret_cast<uintptr_t>(out) % 4 == 0);
     const uint32_t quads = vec ? n / 4 : 0;
     const uint32_t work = quads + (n - 4 * quads);
-    static const unsigned cap = tone_grid_cap();
+    static const unsigned caps[2] = {tone_grid_cap<false>(), tone_grid_cap<true>()};
+    const unsigned cap = caps[vec ? 1 : 0];
     // as many blocks as give every thread the same number of turns
     const uint64_t turns = (static_cast<uint64_t>(work) + static_cast<uint64_t>(cap) * kToneBlock - 1) /
                            (static_cast<uint64_t>(cap) * kToneBlock);
@@ -284,14 +310,14 @@ cudaError_t launch_tonemap_srgb8(const float* rgb, uint8_t* out, uint32_t n, cud
     early.val.programmaticStreamSerializationAllowed = 1;
     if (beside) {
         // a captured launch stays a plain node
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-        else if (cap == cudaStreamCaptureStatusNone) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+        else if (capture == cudaStreamCaptureStatusNone) {
             cfg.attrs = &early;
             cfg.numAttrs = 1;
         }
     }
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_tonemap_srgb8, rgb, out, n, quads, device_table(),
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, vec ? k_tonemap_srgb8<true> : k_tonemap_srgb8<false>, rgb, out, n, quads, device_table(),
                                              float_bits(srgb_table().c_max));
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
