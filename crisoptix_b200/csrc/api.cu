@@ -14,14 +14,12 @@
 #include <vector>
 
 #include "bvh_device.h"
+#include "device_memory.h"
 #include "passes.cuh"
 #include "radix_sort.h"
 #include "records.cuh"
 
 namespace crisb {
-// search.cu: gives back what the endpoint search keeps in the current context
-void trim_search_workspace();
-
 namespace {
 
 thread_local std::string g_last_error;
@@ -74,13 +72,7 @@ struct DevBuf {
     void alloc(size_t count) {
         release();
         if (count == 0) count = 1;
-        cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-        if (e == cudaErrorMemoryAllocation) {  // again without what the endpoint search keeps
-            cudaGetLastError();
-            trim_search_workspace();
-            e = cudaMalloc(&p, count * sizeof(T));
-        }
-        check(e, "cudaMalloc");
+        check(device_malloc(reinterpret_cast<void**>(&p), count * sizeof(T)), "cudaMalloc");
         n = count;
     }
     void upload(const T* src, size_t count) {

@@ -5,6 +5,7 @@
 #include <cfloat>
 #include <cstring>
 
+#include "device_memory.h"
 #include "radix_sort.h"
 
 namespace crisb {
@@ -578,7 +579,7 @@ __global__ void k_qcollapse_write(const int* __restrict__ level, uint32_t nl, co
 
 template <class T>
 cudaError_t dev_alloc(T** p, size_t count) {
-    return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
+    return device_malloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
 }
 
 }  // namespace
@@ -647,8 +648,8 @@ cudaError_t build_wide_bvh_device(const float* pos, uint32_t n, int leaf_max, fl
     TRY(dev_alloc(&kpos, m));
     TRY(dev_alloc(&totals, 4));
     TRY(dev_alloc(&cb, 8));
-    TRY(cudaMalloc(&sort_temp, sort_bytes));
-    TRY(cudaMalloc(&scan_temp, rsort::scan_temp_bytes(m)));
+    TRY(device_malloc(&sort_temp, sort_bytes));
+    TRY(device_malloc(&scan_temp, rsort::scan_temp_bytes(m)));
     auto scan = [&](const uint32_t* in, uint32_t* o, uint32_t cnt, uint32_t* total) {
         return rsort::exclusive_scan(in, o, cnt, total, scan_temp, st);
     };

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "context.h"
+#include "device_memory.h"
 #include "knn.cuh"
 #include "radix_sort.h"
 
@@ -298,7 +299,8 @@ cudaError_t workspace_alloc(void** p, size_t bytes, cudaStream_t st) {
         const RelaxedCapture relaxed;
         if (cudaMemPoolTrimTo(pool, 2 * bytes) != cudaSuccess) cudaGetLastError();
     }
-    const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    const cudaError_t e =
+        alloc_or_trim([&] { return cudaMallocFromPoolAsync(p, bytes, pool, st); }, trim_search_workspace);
     if (e == cudaSuccess) return e;
     cudaGetLastError();
     return cudaMallocAsync(p, bytes, st);
@@ -311,6 +313,7 @@ void trim_search_workspace() {
     std::lock_guard<std::mutex> lock(g_pool_mutex);
     unsigned long long ctx = 0;
     if (g_pools.empty() || current_context_id(&ctx) != cudaSuccess) return;
+    const RelaxedCapture relaxed;
     for (const auto& p : g_pools)
         if (p.first == ctx && p.second && cudaMemPoolTrimTo(p.second, 0) != cudaSuccess) cudaGetLastError();
 }

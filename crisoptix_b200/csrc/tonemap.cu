@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "context.h"
+#include "device_memory.h"
 #include "passes.cuh"
 
 namespace crisb {
@@ -261,7 +262,7 @@ const uint32_t* device_table() {
     void* p = nullptr;
     const std::vector<uint32_t> words = bucket_words(srgb_table());
     const size_t bytes = words.size() * sizeof(uint32_t);
-    if (cudaMalloc(&p, bytes) != cudaSuccess) throw std::runtime_error("sRGB table allocation");
+    if (device_malloc(&p, bytes) != cudaSuccess) throw std::runtime_error("sRGB table allocation");
     if (cudaMemcpy(p, words.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaFree(p);
         throw std::runtime_error("sRGB table upload");
