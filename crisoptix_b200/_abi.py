@@ -240,6 +240,7 @@ ENTRY_POINTS = {
     "crisb_endpoint_search": (c_i32, [c_vp, c_u32, c_vp, c_u32, c_u32, c_vp, c_vp, c_vp]),
     "crisb_endpoint_search_noalloc": (c_i32, [c_vp, c_u32, c_vp, c_u32, c_u32, c_vp, c_vp, c_vp]),
     "crisb_endpoint_search_status": (c_i32, [c_vp]),
+    "crisb_endpoint_search_release": (c_i32, []),
     "crisb_endpoint_search_set_visit_cap": (c_i32, [c_u32]),
     "crisb_selftest_kat": (c_i32, [c_i32, c_vp, c_u32, c_vp, c_vp]),
     "crisb_selftest_sort": (c_i32, [c_vp, c_vp, c_u32, c_vp, ctypes.c_size_t, c_vp]),

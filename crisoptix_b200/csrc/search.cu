@@ -248,8 +248,9 @@ namespace {
 // between calls up to kKeepBytes.  The default pool gives its memory back whenever
 // the device is waited for, and a search then spent 0.8 of 1.25 ms (262,144 entries)
 // reserving it again.  Pool allocations are safe from any thread and on any stream;
-// memory out of proportion to a call goes back before it, all of it when a scene is
-// destroyed or the library runs out of memory (trim_search_workspace).
+// memory out of proportion to a call goes back before it, all of it when the caller
+// says so, a scene is destroyed or the library runs out of memory
+// (trim_search_workspace).
 constexpr uint64_t kKeepBytes = 512ull << 20;
 
 // pool management touches no stream: allowed while another thread captures one
@@ -428,6 +429,11 @@ extern "C" int crisb_endpoint_search_status(void* stream) {
                                 ((word & kDevErrKnn) ? "visit cap" : "") +
                                 ((word & kDevErrKnn) && (word & kDevErrStack) ? ", " : "") +
                                 ((word & kDevErrStack) ? "stack depth" : "") + "); its neighbour list is incomplete");
+    return CRISB_OK;
+}
+
+extern "C" int crisb_endpoint_search_release(void) {
+    crisb::trim_search_workspace();
     return CRISB_OK;
 }
 

@@ -450,8 +450,9 @@ int crisb_trace_rays(const crisb_scene* scene, const float* rays_dev,
  * (distance, entry index), unused slots zeroed; count_dev[q] their number.
  * k in [1, 31].  out_dev and count_dev must be 4-byte aligned.
  * Scratch comes from a stream-ordered pool of the library (up to 512 MiB stay
- * reserved for the next call, until a scene is destroyed; in a captured call,
- * from the graph's own memory); the call is asynchronous.  A query that hits
+ * reserved for the next call, until crisb_endpoint_search_release or the end
+ * of a scene; in a captured call, from the graph's own memory); the call is
+ * asynchronous.  A query that hits
  * the traversal's visit cap or stack depth keeps the neighbours found so far
  * and marks the search error word, which crisb_endpoint_search_status reads
  * (the reference's OptiX query has no such cap and reports nothing). */
@@ -467,6 +468,11 @@ int crisb_endpoint_search(const float* entries_dev, uint32_t n_entries,
  * allocator.  The renderer's own searches report through
  * crisb_check_device_errors instead. */
 int crisb_endpoint_search_status(void* stream);
+
+/* Gives back the device memory that crisb_endpoint_search keeps reserved in
+ * the current CUDA context between calls (memory that searches still running
+ * use stays).  Safe from any thread.  No counterpart in the reference. */
+int crisb_endpoint_search_release(void);
 
 /* Test hook: caps the node visits of each standalone search query at
  * max_visits (0 restores the default cap of 2^21).  Process-wide. */
