@@ -503,7 +503,9 @@ int validate_qbvh(const std::vector<Bvh8QNode>& nodes, const std::vector<uint32_
             for (int a = 0; a < 3; ++a) {
                 const double lo = p[a] + std::ldexp(static_cast<double>(qlo[a][c]), e[a]);
                 const double hi = p[a] + std::ldexp(static_cast<double>(qhi[a][c]), e[a]);
+                const double in = std::ldexp(kQRounding, e[a]);  // what the slab test may lose
                 if (lo > cb[a] - half || hi < cb[3 + a] + half) fail("child box does not contain its subtree");
+                if (lo + in > cb[a] - half || hi - in < cb[3 + a] + half) fail("child box without slack");
                 box[a] = std::min(box[a], cb[a]);
                 box[3 + a] = std::max(box[3 + a], cb[3 + a]);
             }

@@ -81,12 +81,17 @@ constexpr int kQTrisPerNode = 24;  // triangles per compressed node
 // per-node terms stay finite for every ray direction; larger scenes use
 // 4-wide nodes)
 constexpr float kQMaxCoord = 1.6e7f;
+// The slab test rounds a node's plane offsets (qnode_test): a plane may be met up to
+// kQRounding grid steps early or late.  The builder keeps kQSlack steps free around
+// every child box.
+constexpr double kQRounding = 0.001953125;  // 2^-9
+constexpr double kQSlack = 0.0078125;       // 2^-7
 
 // Structural check of a compressed tree: node links in range and each node
 // reached once, leaves of 1-3 triangles inside the node's 24, every triangle
-// in exactly one leaf, every decoded child box containing its subtree's
-// triangles widened by half the margin (compared in double precision), grid
-// exponents in range.  `order`: leaf order -> triangle.  Returns the depth of
+// in exactly one leaf, every decoded child box, taken in by kQRounding grid
+// steps, containing its subtree's triangles widened by half the margin
+// (compared in double precision), grid exponents in range.  `order`: leaf order -> triangle.  Returns the depth of
 // the tree (the traversal's group-stack bound).  Throws std::runtime_error.
 int validate_qbvh(const std::vector<Bvh8QNode>& nodes, const std::vector<uint32_t>& order, const float* pos,
                   uint32_t num_tris, float margin);

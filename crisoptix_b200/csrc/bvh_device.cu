@@ -461,10 +461,6 @@ __global__ void k_dp_count(const int* __restrict__ level, uint32_t nl, const BNo
 // first, cost = centroid offset from the node's centre along the slot's
 // diagonal, ties to the lower child then slot), boxes widened by `margin`
 // then quantised outward in double precision
-// kQSlack: grid steps kept free around every child box, for the rounding of
-// the traversal's plane offsets (qnode_test)
-constexpr double kQSlack = 0.0078125;
-
 __global__ void k_qcollapse_write(const int* __restrict__ level, uint32_t nl, const BNode* __restrict__ nodes,
                                   uint32_t n_tris, const uint32_t* __restrict__ order, const float* __restrict__ pos,
                                   const uint32_t* __restrict__ inner_off, const uint32_t* __restrict__ tri_off,
