@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "adjoint_common.cuh"
+#include "queues.cuh"
 
 namespace crisb {
 namespace {
@@ -266,23 +267,12 @@ __global__ void __launch_bounds__(kGroup, 5) k_frozen_backward(AdjView a, FrameP
     }
 }
 
-// blocks of `kernel` resident on the device at once
-unsigned resident_blocks(const void* kernel) {
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPassBlock, 0) == cudaSuccess && sms > 0 &&
-        per_sm > 0)
-        return static_cast<unsigned>(sms * per_sm);
-    return 148u * 4u;
-}
-
 template <int kFmt>
 void forward(const SceneView& eval, const crisb_material* sample_mats, uint32_t num_mats, const FrameParams& fp,
              float* out, cudaStream_t st) {
     const AdjView a{eval, sample_mats, num_mats, eval.num_emitters};
     const uint32_t P = fp.width * fp.height;
-    static const unsigned resident = resident_blocks(reinterpret_cast<const void*>(k_frozen_forward<kFmt>));
+    static const unsigned resident = persistent_grid(reinterpret_cast<const void*>(k_frozen_forward<kFmt>));
     k_frozen_forward<kFmt><<<std::min((P + kPassBlock - 1) / kPassBlock, resident), kPassBlock, 0, st>>>(a, fp, out);
 }
 
@@ -295,7 +285,7 @@ void backward(const SceneView& eval, const crisb_material* sample_mats, uint32_t
     const int use_shared = sh_bytes <= kSharedGradBytes ? 1 : 0;
     const size_t shb = use_shared ? sh_bytes : 0;
     allow_shared_grads(reinterpret_cast<const void*>(k_frozen_backward<kFmt>), shb);
-    static const unsigned resident = resident_blocks(reinterpret_cast<const void*>(k_frozen_backward<kFmt>));
+    static const unsigned resident = persistent_grid(reinterpret_cast<const void*>(k_frozen_backward<kFmt>));
     const unsigned groups = (P + kGroup - 1) / kGroup;
     const unsigned threads = groups <= resident ? kGroup : kGroupThreads;
     k_frozen_backward<kFmt><<<groups, threads, shb, st>>>(a, fp, d_img, g_mat, g_em, use_shared);

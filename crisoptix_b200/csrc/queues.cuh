@@ -109,21 +109,10 @@ __global__ void __launch_bounds__(kB, TraceShape<kB>::kMinBlocks) k_q_trace(Scen
     }
 }
 
-// all blocks of `kernel` that are resident on the device at once
-inline unsigned persistent_grid(const void* kernel) {
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPassBlock, 0) == cudaSuccess && sms > 0 &&
-        per_sm > 0)
-        return static_cast<unsigned>(sms * per_sm);
-    return 148u * 4u;
-}
-
 inline unsigned grid_for(uint32_t n) { return (n + kPassBlock - 1) / kPassBlock; }
 
-// all blocks of `kernel` at `block` threads resident on the device at once
-inline unsigned persistent_grid_at(const void* kernel, int block) {
+// all blocks of `kernel` at `block` threads that are resident on the device at once
+inline unsigned persistent_grid(const void* kernel, int block = kPassBlock) {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
@@ -135,7 +124,7 @@ inline unsigned persistent_grid_at(const void* kernel, int block) {
 
 template <class R, int kB, int kFmt>
 unsigned trace_grid_of() {
-    static const unsigned g = persistent_grid_at(reinterpret_cast<const void*>(k_q_trace<R, kB, kFmt>), kB);
+    static const unsigned g = persistent_grid(reinterpret_cast<const void*>(k_q_trace<R, kB, kFmt>), kB);
     return g;
 }
 

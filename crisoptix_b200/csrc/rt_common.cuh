@@ -30,7 +30,6 @@ struct V3 {
     float x, y, z;
 };
 
-RT_HD V3 mk(float x, float y, float z) { return V3{x, y, z}; }
 RT_HD V3 splat(float s) { return V3{s, s, s}; }
 RT_HD V3 operator+(V3 a, V3 b) { return V3{a.x + b.x, a.y + b.y, a.z + b.z}; }
 RT_HD V3 operator-(V3 a, V3 b) { return V3{a.x - b.x, a.y - b.y, a.z - b.z}; }
@@ -59,7 +58,6 @@ RT_HD float gclamp(float x, float lo, float hi) { return gmin(gmax(x, lo), hi); 
 RT_HD bool nonfinite(float v) { return isnan(v) || isinf(v); }
 RT_HD bool nonfinite(V3 v) { return nonfinite(v.x) || nonfinite(v.y) || nonfinite(v.z); }
 RT_HD bool is_zero(V3 v) { return v.x == 0.0f && v.y == 0.0f && v.z == 0.0f; }
-RT_HD float comp(V3 v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : v.z); }
 RT_HD V3 ld3(const float* p) { return V3{p[0], p[1], p[2]}; }
 RT_HD void st3(float* p, V3 v) {
     p[0] = v.x;
@@ -321,11 +319,9 @@ RT_HD void st_prefix(crisb_prefix_rec& r, const Prefix& p) {
     r.path_len = p.path_len;
     st3(r.recon_out_dir, p.rod);
 }
-// The prefix record as eight 16-byte words (the same bytes as the field-wise
-// forms above; records of the device arrays start 16-byte aligned): a whole
-// record in 8 memory instructions instead of ~25, and the running values a
-// path-machine step moves (flags, f, postReconF, p, path length, reconOutDir)
-// in the last three words.
+// The prefix record read as eight 16-byte words (the same bytes as the
+// field-wise forms above; records of the device arrays start 16-byte aligned): a
+// whole record in 8 memory instructions instead of ~25.
 static_assert(sizeof(crisb_prefix_rec) == 128 && offsetof(crisb_prefix_rec, primary) == 8 &&
                   offsetof(crisb_prefix_rec, recon) == 32 && offsetof(crisb_prefix_rec, last) == 56 &&
                   offsetof(crisb_prefix_rec, flags) == 80 && offsetof(crisb_prefix_rec, f) == 84 &&
@@ -336,26 +332,8 @@ static_assert(sizeof(crisb_hit_rec) == 24 && offsetof(crisb_hit_rec, bary) == 4 
                   offsetof(crisb_hit_rec, in_dir) == 12,
               "hit record layout");
 #ifdef __CUDACC__
-__device__ inline uint32_t fbits(float v) { return __float_as_uint(v); }
 __device__ inline float bitsf(uint32_t v) { return __uint_as_float(v); }
-// words 5-7: flags, f, postReconF, p, path length, reconOutDir
-__device__ inline void ld_prefix_tail_v(const crisb_prefix_rec& r, Prefix& p) {
-    const uint4* w = reinterpret_cast<const uint4*>(&r);
-    const uint4 a = w[5], b = w[6], c = w[7];
-    p.flags = a.x;
-    p.f = V3{bitsf(a.y), bitsf(a.z), bitsf(a.w)};
-    p.prf = V3{bitsf(b.x), bitsf(b.y), bitsf(b.z)};
-    p.p = bitsf(b.w);
-    p.path_len = bitsf(c.x);
-    p.rod = V3{bitsf(c.y), bitsf(c.z), bitsf(c.w)};
-}
-__device__ inline void st_prefix_tail_v(crisb_prefix_rec& r, const Prefix& p) {
-    uint4* w = reinterpret_cast<uint4*>(&r);
-    w[5] = make_uint4(p.flags, fbits(p.f.x), fbits(p.f.y), fbits(p.f.z));
-    w[6] = make_uint4(fbits(p.prf.x), fbits(p.prf.y), fbits(p.prf.z), fbits(p.p));
-    w[7] = make_uint4(fbits(p.path_len), fbits(p.rod.x), fbits(p.rod.y), fbits(p.rod.z));
-}
-// the record's eight words from / to the fields
+// the fields of the record's eight words
 __device__ inline Prefix prefix_of_words(const uint4 (&w)[8]) {
     const uint4 a = w[0], b = w[1], c = w[2], d = w[3], e = w[4], f = w[5], g = w[6], h = w[7];
     Prefix p;
@@ -371,30 +349,12 @@ __device__ inline Prefix prefix_of_words(const uint4 (&w)[8]) {
     p.rod = V3{bitsf(h.y), bitsf(h.z), bitsf(h.w)};
     return p;
 }
-__device__ inline void words_of_prefix(const Prefix& p, uint4 (&w)[8]) {
-    w[0] = make_uint4(static_cast<uint32_t>(p.rng), static_cast<uint32_t>(p.rng >> 32), p.primary.prim,
-                      fbits(p.primary.bu));
-    w[1] = make_uint4(fbits(p.primary.bv), fbits(p.primary.dir.x), fbits(p.primary.dir.y), fbits(p.primary.dir.z));
-    w[2] = make_uint4(p.recon.prim, fbits(p.recon.bu), fbits(p.recon.bv), fbits(p.recon.dir.x));
-    w[3] = make_uint4(fbits(p.recon.dir.y), fbits(p.recon.dir.z), p.last.prim, fbits(p.last.bu));
-    w[4] = make_uint4(fbits(p.last.bv), fbits(p.last.dir.x), fbits(p.last.dir.y), fbits(p.last.dir.z));
-    w[5] = make_uint4(p.flags, fbits(p.f.x), fbits(p.f.y), fbits(p.f.z));
-    w[6] = make_uint4(fbits(p.prf.x), fbits(p.prf.y), fbits(p.prf.z), fbits(p.p));
-    w[7] = make_uint4(fbits(p.path_len), fbits(p.rod.x), fbits(p.rod.y), fbits(p.rod.z));
-}
 __device__ inline Prefix ld_prefix_v(const crisb_prefix_rec& r) {
     const uint4* s = reinterpret_cast<const uint4*>(&r);
     uint4 w[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) w[k] = s[k];
     return prefix_of_words(w);
-}
-__device__ inline void st_prefix_v(crisb_prefix_rec& r, const Prefix& p) {
-    uint4 w[8];
-    words_of_prefix(p, w);
-    uint4* d = reinterpret_cast<uint4*>(&r);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) d[k] = w[k];
 }
 #endif
 

@@ -156,24 +156,6 @@ RT_HD bool intersect_tri(const RayPre& r, V3 p0, V3 p1, V3 p2, float tmin, float
     return true;
 }
 
-RT_D bool slab(const RayPre& r, float lox, float loy, float loz, float hix, float hiy, float hiz, float tmin,
-               float tmax, float& tnear) {
-    float t0 = (lox - r.org.x) * r.inv.x, t1 = (hix - r.org.x) * r.inv.x;
-    float tn = fminf(t0, t1), tf = fmaxf(t0, t1);
-    t0 = (loy - r.org.y) * r.inv.y;
-    t1 = (hiy - r.org.y) * r.inv.y;
-    tn = fmaxf(tn, fminf(t0, t1));
-    tf = fminf(tf, fmaxf(t0, t1));
-    t0 = (loz - r.org.z) * r.inv.z;
-    t1 = (hiz - r.org.z) * r.inv.z;
-    tn = fmaxf(tn, fminf(t0, t1));
-    tf = fminf(tf, fmaxf(t0, t1));
-    tn = fmaxf(tn, tmin);
-    tf = fminf(tf, tmax);
-    tnear = tn;
-    return tn <= tf * kSlabFarScale;
-}
-
 struct TraceResult {
     uint32_t prim;  // CRISB_INVALID_PRIM: miss
     float t, u, v;
@@ -231,8 +213,8 @@ struct Trav {
 
     RT_D float bound() const { return best.prim == CRISB_INVALID_PRIM ? tmax : best.t; }
 
-    // slab() with the near / far plane of each axis chosen by the sign of the
-    // inverse direction: the same values as the min / max form, since
+    // The near / far plane of each axis is chosen by the sign of the inverse
+    // direction: the same values as the min / max of both planes' t, since
     // (lo - o) * inv <= (hi - o) * inv exactly when inv > 0 (rounding is
     // monotonic) and the inverse direction is never zero or NaN.  (One FMA per
     // plane against a per-ray org * inv measured no faster: 13.67 against

@@ -21,7 +21,6 @@
 namespace crisb {
 namespace {
 
-RT_D V3 f3(float4 v) { return V3{v.x, v.y, v.z}; }
 RT_D float4 f4(V3 v, float w) { return make_float4(v.x, v.y, v.z, w); }
 
 enum WfPhase : uint32_t {
