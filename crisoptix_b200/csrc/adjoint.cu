@@ -1,7 +1,7 @@
 // adjoint.cu -- path-replay adjoint of the unidirectional path tracer.
 //
 // The estimator differentiated is TraceCompletePath
-// (include/graph/restir/path_gen.h:389-472; trace_complete_path here) with its
+// (include/graph/restir/path_gen.h:389-472; CompletePath here) with its
 // sampling frozen: every random decision, BRDF-sampled direction and sampling
 // pdf comes from a fixed copy of the materials (theta0, taken when the adjoint
 // context is made), while the BRDF values, emissions and emitter colours come

@@ -101,10 +101,10 @@ struct Bufs {
     uint32_t* path_counts;       // 2 per round (Counters)
     uint32_t* path_next;         // 1 (Counters)
     crisb_prefix_rec* gather_cp; // canonical prefix of the final gather
-    // shift machines: one record per job of the list, ray queues of two
+    // shift machines: a record per job of the list up to job_cap, ray queues of two
     // rounds (closest, shadow) x 2 and the counts of every round of the phase
-    ShiftJob* jobs;         // P * slots
-    uint32_t* job_queue[4]; // P * slots each
+    ShiftJob* jobs;         // job_cap
+    uint32_t* job_queue[4]; // job_cap each
     uint32_t* job_qcount;   // 2 per round (Counters)
     uint32_t* job_next;     // 1: next item of the persistent launch (Counters)
 

@@ -24,13 +24,13 @@
 // expectation's gradient is the expectation of its gradient (W_n are unbiased
 // contribution weights and the MIS weights sum to one whatever the integrand).
 //
-// Nothing is taped: each factor is re-traced.  The canonical prefix from the
-// camera along its stored primary direction with its stored random state, the
-// canonical suffix from the prefix's last vertex with its stored state, the
-// shift from the stored neighbour sample, and R_n from the neighbour sample's
-// own seed: its random state advanced four draws per suffix vertex (one NEE
-// decision, three for BRDF sampling) to the vertex after its reconnection
-// vertex, whose loop index the suffix flags carry (bits 24-31).  Forward mode
+// Nothing is taped: each factor is re-traced.  The canonical prefix from its
+// stored primary hit with its stored random state, the canonical suffix from
+// the prefix's last vertex with its stored state, the shift from the stored
+// neighbour sample, and R_n from the neighbour sample's own seed: its random
+// state advanced four draws per suffix vertex (one NEE decision, three for
+// BRDF sampling) to the vertex after its reconnection vertex, whose loop index
+// the suffix flags carry (bits 24-31).  Forward mode
 // carries d(throughput)/d(diffuse, roughness) per material met, d/d(colour) of
 // the emitter sampled and d/d(emission); the backward kernel weighs each
 // factor's derivatives with dLoss/dL times the other factors (chain rule at

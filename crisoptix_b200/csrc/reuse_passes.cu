@@ -448,8 +448,8 @@ __global__ void __launch_bounds__(kPassBlock) k_suffix_temp_finish(FrameParams f
 // latency-bound, and more warps in flight beat the spills (0.935 -> 0.902 ms
 // per 1080p frame; 12 and 16 blocks spill more: 0.995 and 1.23 ms).  Their
 // reservoir stores stay per thread: storing a warp's records as one run
-// through shared memory (as the path-machine init kernels do) took 0.895 ->
-// 1.09 ms, the kernels having to reach the store with every lane.
+// through shared memory took 0.895 -> 1.09 ms, the kernels having to reach the
+// store with every lane.
 constexpr int kResampleMinBlocks = 10;
 
 __global__ void __launch_bounds__(kPassBlock, kResampleMinBlocks) k_suffix_temp_combine(FrameParams fp, Bufs b) {
@@ -1011,8 +1011,11 @@ RT_D void prefix_tail(const FrameParams& fp, const Bufs& b, float* out, uint32_t
 // Persistent warps whose lanes take the next pixel as their paths end, one ray of
 // either kind per lane and turn: 1.87 -> 1.15 ms for a 960x540 frame of the large
 // scene against a thread a pixel (2.0 G rays/s).  4 / 5 / 6 / 7 resident blocks
-// (115, 94, 80, 72 registers): 1.25 / 1.15 / 1.13 / 1.19 ms; refilling only once 8 or
-// 16 lanes are idle: 1.15 / 1.23 ms.
+// (117, 94, 80, 72 registers): 1.261 / 1.126 / 1.133 / 1.194 ms; the room at 160x120
+// 244 / 247 / 253 / 256 us, at 1080p 4.23 / 3.97 / 3.91 / 3.93 ms, at 640x360 with paths
+// of up to 30 vertices 1.042 / 0.985 / 1.033 / 1.076 ms.  Only the boxes at 1080p, whose
+// traversals are short, want more warps (textured 2.43 / 2.27 / 2.00 / 1.76 ms).
+// Refilling only once 8 or 16 lanes are idle: 1.15 / 1.23 ms, 1.15 without.
 template <bool kTex, int kFmt>
 __global__ void __launch_bounds__(kPassBlock, 5) k_path_tracer(SceneView s, FrameParams fp, float* out) {
     PixelPool pool(pixel_count(fp));
@@ -1194,7 +1197,8 @@ const ShiftGrids& shift_grids() {
 // ones 2.29 against 2.35; at 641x479 textured jobs that replay long prefixes, two
 // to a lane, take 1.17 against 0.67), one above (960x540 4.45 ms against 4.54 with
 // none, 4.74 with two, 4.91 with three; 1080p 14.0 against 15.0, 14.0, 14.3), two
-// for views that render beside one another (16 views: 76.0 ms, 78.3 with one).
+// for views that render beside one another (16 views: 76.0 ms, 78.3 with one; smaller
+// batches: flow_rounds).
 // Three rounds whose last step traced the rays left in place, a thread a job, took
 // 4.95 and 14.3 ms.
 int shift_rounds(const FrameParams& fp) {

@@ -186,7 +186,13 @@ void launch_flow(const SceneView& s, const FrameParams& fp, const Bufs& b, cudaS
 // (4.95 ms, 5.03 with one more each), two and three at 1080p (14.31 ms, 14.47 and
 // 14.55 with one fewer and one more); views that render beside one another fill
 // each other's late rounds, so theirs go on longest (16 views 75.9 ms, 78.7 with
-// the single view's rounds).  By rounds to the last ray, the three flows of a
+// the single view's rounds).  That line is drawn for batches that fill the GPU (8 views
+// of 512x512 12.5 ms, 13.3 with 2 / 2 / 3 rounds and one of shifts, 14.0 with 1 / 1 / 2,
+// 17.0 with none; two of 1080p 24.5, 25.0, 25.4, 31.5).  Around a million pixels it makes
+// no difference (4 of 512x512 7.05, 7.05, 7.45, 8.89), and smaller batches would run
+// faster with fewer: 2 of 256x256 2.82, 2.47, 2.40, 2.24, 16 of 64x64 2.24, 1.98, 1.89,
+// 1.53.  (With rounds to the last ray these four took 15.4, 8.92, 3.80 and 5.74, the
+// 1080p pair 29.8.)  By rounds to the last ray, the three flows of a
 // 1080p frame took 0.5 ms more, those of a 960x540 frame 0.4.
 int flow_rounds(const FrameParams& fp, int flow, bool textured) {
     const uint32_t pixels = fp.width * fp.height;
