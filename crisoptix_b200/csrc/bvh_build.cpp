@@ -477,7 +477,7 @@ int validate_qbvh(const std::vector<Bvh8QNode>& nodes, const std::vector<uint32_
         const Bvh8QNode& nd = nodes[v];
         double box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
         const double p[3] = {nd.px, nd.py, nd.pz};
-        const int e[3] = {nd.ex, nd.ey, nd.ez};
+        const double step[3] = {std::ldexp(1.0, nd.ex), std::ldexp(1.0, nd.ey), std::ldexp(1.0, nd.ez)};
         const uint8_t* qlo[3] = {nd.qlo_x, nd.qlo_y, nd.qlo_z};
         const uint8_t* qhi[3] = {nd.qhi_x, nd.qhi_y, nd.qhi_z};
         int rank = 0;
@@ -501,9 +501,9 @@ int validate_qbvh(const std::vector<Bvh8QNode>& nodes, const std::vector<uint32_
                 }
             }
             for (int a = 0; a < 3; ++a) {
-                const double lo = p[a] + std::ldexp(static_cast<double>(qlo[a][c]), e[a]);
-                const double hi = p[a] + std::ldexp(static_cast<double>(qhi[a][c]), e[a]);
-                const double in = std::ldexp(kQRounding, e[a]);  // what the slab test may lose
+                const double lo = p[a] + qlo[a][c] * step[a];
+                const double hi = p[a] + qhi[a][c] * step[a];
+                const double in = kQRounding * step[a];  // what the slab test may lose
                 if (lo > cb[a] - half || hi < cb[3 + a] + half) fail("child box does not contain its subtree");
                 if (lo + in > cb[a] - half || hi - in < cb[3 + a] + half) fail("child box without slack");
                 box[a] = std::min(box[a], cb[a]);
