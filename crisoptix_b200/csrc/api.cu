@@ -138,7 +138,9 @@ RT_D int direction_exponent(float x, float y, float z) {
 // differ in nodes and triangles).  8 resident blocks per SM (64 registers): a million
 // camera and bounce rays, nearest hits and occlusion, take 716 us against 755 with
 // 67-72 registers, 8-word scalar loads and one kernel for both queries; 6 / 7 / 9 / 10
-// blocks 785 / 741 / 727 / 765.
+// blocks 785 / 741 / 727 / 765.  (The rescaling of long and short directions holds a
+// register during a nearest-hit traversal: 1.5% of it.  Out of line, or with the exponent
+// in shared memory, other forms of the kernel lost as much.)
 template <bool kAny, bool kVec>
 __global__ void __launch_bounds__(kPassBlock, 8) k_trace_rays(SceneView s, const float* rays, crisb_trace_hit* hits,
                                                              uint32_t n) {
